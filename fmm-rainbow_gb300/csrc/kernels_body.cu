@@ -440,21 +440,102 @@ __global__ void __launch_bounds__(256, 6) k_integrate(const SceneDesc *__restric
 //
 // Exact softened pair sums of every body over the bodies of the 3x3x3 cells
 // around its sample cell (kNearP2P), written per slot for the integrate that
-// follows.  Persistent CTAs walk interleaved tiles of 256 leaf-sorted bodies.
-// A tile whose bodies all share one sample cell (the common case: a dense
-// leaf holds thousands of bodies) stages its 27 cells' sources as coalesced
-// float4 chunks in shared memory and every thread reads each source by
-// broadcast; otherwise each warp whose bodies share a sample cell does the
-// same with its own 32-source slice, and the remaining bodies gather their
-// sources themselves.  Every thread sums in the same fixed order (cells z-,
-// y-, x-major, bodies in slot order, itself skipped) whichever way its
-// sources arrive, so the sums equal p2p_sums bit for bit under the exact
-// contract.
+// follows.  What bounds it is the FP32 pipe: 23 operations per pair in the
+// exact contract, 11 in the fast variant, with packed three-operand
+// multiply-adds at 3.2 instead of 2 cycles (measured: their register reads)
+// about 29 and 13 cycles per warp and source.
+//
+// Warps work alone: a warp takes kUnit consecutive leaf-sorted slots from a
+// counter, so the expensive core regions spread over every SM sub-partition
+// (a CTA per 256 slots left most of them idle at 120,001 bodies).  Lanes
+// 0..26 look up the 27 neighbour ranges at once; their sources form one
+// sequence (cells z-, y-, x-major, bodies in slot order) that the warp stages
+// in chunks of kP2PChunk as x, y and z rows in shared memory, two sources to
+// a packed operation (the packed forms keep each half's rounding and save
+// issue slots).  The next chunk's loads are in flight meanwhile.  A warp
+// whose bodies sample several cells does one cell after the other.
+//
+// The exact variant adds every term in that order, so the sums equal
+// p2p_sums bit for bit.  The body itself and the padding of the last chunk
+// add +0, which changes no sum (sums start at +0 and never become -0).  The
+// inner loop has no range check: it runs when every source of the chunk lies
+// within 2^60, every body of the warp within 2^59 and softening^2 between
+// 2^-80 and 2^120, so that 2^-80 <= r^2 < 2^127 and a padding term underflows
+// to +0; otherwise (non-finite or astronomically distant bodies, no
+// softening) p2p_chunk_checked evaluates the plain expressions.
+//
+// kSplit lanes share a body: each evaluates its share of the sources.  The
+// fast variant sums the shares at the end.  In the exact variant the terms
+// cross through shared memory and lane c of a body's lanes adds component c
+// in order.  A cell holding one of the warp's bodies is summed by all 32
+// lanes, one holding up to eight by four lanes each (outlying bodies share a
+// warp with few of their cell's but have up to every body of the scene as a
+// source: one such warp used to end the launch).
+//
+// Measured, ms per launch, one CTA per 256 slots with IEEE 1/sqrt before ->
+// now: Plummer 1,048,576 exact 167 -> 108, fast 88 -> 60; Plummer 120,001
+// exact 50 -> 8.8; clusters 600,007 fast 26 -> 15.
+
+constexpr uint32_t kP2PChunk = 128u;       // sources per staged chunk: four per lane
+constexpr uint32_t kP2PWarps = 4u;         // warps per CTA (independent)
+constexpr float kP2PFar = 0x1p60f;         // padding coordinate: its term underflows to +0
+#ifdef RFMM_FAST_FLOAT
+constexpr uint32_t kP2PBodies = 2u;        // bodies per lane
+#else
+constexpr uint32_t kP2PBodies = 1u;
+#endif
+template <uint32_t kSplit>
+constexpr uint32_t kP2PUnit = 32u / kSplit * kP2PBodies;  // slots per work unit
+// Two binary32 values in a 64-bit register pair; every operation rounds each
+// half to nearest.
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+  f32x2 v;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+  return v;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float &lo, float &hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+// RN(a b) as a b + (-0), signed zeros included; `mz` holds two -0 the
+// compiler cannot see through.  (mul.rn.f32x2, or -0 as a constant, feeding an
+// add.rn.f32x2 comes out contracted even under -fmad=false: measured, one r^2
+// in five rounded differently from the scalar expression.)
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b, f32x2 mz) { return fma2(a, b, mz); }
+
+// One warp's staged sources: x, y and z rows of a chunk, and the neighbour
+// ranges as a sequence (first sequence index of each range, and what to add to
+// a sequence index to get its slot).
+struct alignas(16) P2PStage {
+  float x[kP2PChunk], y[kP2PChunk], z[kP2PChunk];
+  uint32_t first[28], shift[27];
+};
+static_assert(sizeof(P2PStage) % 16u == 0u && kP2PChunk % 8u == 0u, "rows are read up to 16 bytes at a time");
+
+// Terms on their way to the adding lanes (exact variant).  kSplit 4: 16
+// sources of body b, component c from kP2PTermBody b + kP2PTermComp c on (the
+// strides put the 16-byte accesses of eight lanes on distinct banks), two
+// buffers in turn; kSplit 32: one row of 128 sources per component.
+constexpr uint32_t kP2PTermBody = 80u, kP2PTermComp = 20u;
+struct alignas(16) P2PTerms {
+  float v[2][8u * kP2PTermBody];
+};
+static_assert(8u * kP2PTermBody >= 3u * kP2PChunk, "kSplit 32 uses one buffer");
 
 // One source's contribution (the expression p2p_sums evaluates).
-__device__ __forceinline__ void p2p_pair(float4 q, float px, float py, float pz, float eps2,
-                                         float &sx, float &sy, float &sz) {
-  const float dx = q.x - px, dy = q.y - py, dz = q.z - pz;
+__device__ __forceinline__ void p2p_pair(float qx, float qy, float qz, float px, float py, float pz,
+                                         float eps2, float &sx, float &sy, float &sz) {
+  const float dx = qx - px, dy = qy - py, dz = qz - pz;
   const float r2 = ((dx * dx + dy * dy) + dz * dz) + eps2;
   const float inv = inv_sqrt(r2);
   const float w = (inv * inv) * inv;
@@ -463,45 +544,65 @@ __device__ __forceinline__ void p2p_pair(float4 q, float px, float py, float pz,
   sz = sz + dz * w;
 }
 
-// Sources [lo, hi) through a staging buffer of kWidth float4 shared by the
-// kWidth threads of a group (a CTA or a warp); `sync` orders the group.
-template <uint32_t kWidth, typename Sync>
-__device__ __forceinline__ void p2p_staged_range(const float4 *__restrict__ pos, uint32_t lo,
-                                                 uint32_t hi, float4 *buf, uint32_t rank,
-                                                 uint32_t self, float px, float py, float pz,
-                                                 float eps2, float &sx, float &sy, float &sz,
-                                                 Sync sync) {
-  for (uint32_t base = lo; base < hi; base += kWidth) {
-    sync();  // the previous chunk is consumed
-    if (base + rank < hi) buf[rank] = __ldg(&pos[base + rank]);
-    sync();
-    const uint32_t m = min(kWidth, hi - base);
-    if (self - base < m) {  // this chunk holds the body itself: skip it
-      for (uint32_t k = 0; k < m; k++)
-        if (base + k != self) p2p_pair(buf[k], px, py, pz, eps2, sx, sy, sz);
-    } else {
-#ifdef RFMM_FAST_FLOAT
-      // Two partial sums (even and odd sources) give each thread two
-      // independent chains; the fast variant does not keep the reference
-      // summation order.
-      float ax = 0.0f, ay = 0.0f, az = 0.0f, bx = 0.0f, by = 0.0f, bz = 0.0f;
-      uint32_t k = 0;
-#pragma unroll 2
-      for (; k + 1u < m; k += 2u) {
-        p2p_pair(buf[k], px, py, pz, eps2, ax, ay, az);
-        p2p_pair(buf[k + 1u], px, py, pz, eps2, bx, by, bz);
-      }
-      if (k < m) p2p_pair(buf[k], px, py, pz, eps2, ax, ay, az);
-      sx = sx + (ax + bx);
-      sy = sy + (ay + by);
-      sz = sz + (az + bz);
-#else
-#pragma unroll 4
-      for (uint32_t k = 0; k < m; k++) p2p_pair(buf[k], px, py, pz, eps2, sx, sy, sz);
-#endif
-    }
-  }
+// Sums of one lane's body over a staged chunk of `m` sources.  `self` is the
+// chunk index of the body itself (anything >= m: not in this chunk).
+__device__ __noinline__ float3 p2p_chunk_checked(const P2PStage &T, uint32_t m, uint32_t self, float px,
+                                                 float py, float pz, float eps2, float3 s) {
+  for (uint32_t k = 0; k < m; k++)
+    if (k != self) p2p_pair(T.x[k], T.y[k], T.z[k], px, py, pz, eps2, s.x, s.y, s.z);
+  return s;
 }
+
+// One body's side of the packed loop: minus its position, twice.
+struct P2PBody {
+  f32x2 nx, ny, nz;
+};
+
+#ifdef RFMM_FAST_FLOAT
+// Even and odd sources of a chunk in the halves of the partial sums.
+__device__ __forceinline__ void p2p_two(f32x2 qx, f32x2 qy, f32x2 qz, const P2PBody &b, f32x2 eps2, f32x2 mz,
+                                        f32x2 &sx, f32x2 &sy, f32x2 &sz) {
+  const f32x2 dx = add2(qx, b.nx), dy = add2(qy, b.ny), dz = add2(qz, b.nz);
+  const f32x2 r2 = fma2(dz, dz, fma2(dy, dy, fma2(dx, dx, eps2)));
+  float x0, x1;
+  unpack2(r2, x0, x1);
+  const f32x2 inv = pack2(rsqrt_estimate(x0), rsqrt_estimate(x1));
+  const f32x2 w = mul2(mul2(inv, inv, mz), inv, mz);
+  sx = fma2(dx, w, sx);
+  sy = fma2(dy, w, sy);
+  sz = fma2(dz, w, sz);
+}
+#else
+// The terms of two consecutive sources; inv_sqrt_in_range in packed form
+// (signs folded into the factors built from y's bit pattern).
+__device__ __forceinline__ void p2p_two(f32x2 qx, f32x2 qy, f32x2 qz, const P2PBody &b, f32x2 eps2, f32x2 mz,
+                                        f32x2 &tx, f32x2 &ty, f32x2 &tz) {
+  const f32x2 dx = add2(qx, b.nx), dy = add2(qy, b.ny), dz = add2(qz, b.nz);
+  const f32x2 r2 = add2(add2(add2(mul2(dx, dx, mz), mul2(dy, dy, mz)), mul2(dz, dz, mz)), eps2);
+  float x0, x1, g0, g1;
+  unpack2(r2, x0, x1);
+  const float y0 = rsqrt_estimate(x0), y1 = rsqrt_estimate(x1);
+  const uint32_t u0 = __float_as_uint(y0), u1 = __float_as_uint(y1);
+  const f32x2 y = pack2(y0, y1);
+  const f32x2 nh = pack2(__uint_as_float(u0 + 0x7F800000u), __uint_as_float(u1 + 0x7F800000u));  // -y/2
+  const f32x2 up = pack2(__uint_as_float(u0 + 1u), __uint_as_float(u1 + 1u));                    // y + ulp
+  const f32x2 ny = pack2(__uint_as_float(u0 ^ 0x80000000u), __uint_as_float(u1 ^ 0x80000000u));  // -y
+  const f32x2 g = mul2(r2, y, mz);
+  unpack2(g, g0, g1);
+  const f32x2 root = fma2(pack2(__fmaf_rn(g0, g0, -x0), __fmaf_rn(g1, g1, -x1)), nh, g);
+  const f32x2 ne = fma2(root, y, pack2(-1.0f, -1.0f));  // -e
+  const f32x2 inv = fma2(ne, fma2(ne, up, ny), y);
+  const f32x2 w = mul2(mul2(inv, inv, mz), inv, mz);
+  tx = mul2(dx, w, mz);
+  ty = mul2(dy, w, mz);
+  tz = mul2(dz, w, mz);
+}
+__device__ __forceinline__ float add_both(float s, f32x2 t) {
+  float a, b;
+  unpack2(t, a, b);
+  return __fadd_rn(__fadd_rn(s, a), b);
+}
+#endif
 
 // Slot range [lo, hi) of neighbour j (0..26, in the reference's z-, y-,
 // x-major order) of cell (cx, cy, cz) at level l; false when j lies outside
@@ -520,14 +621,186 @@ __device__ __forceinline__ bool neighbour_range(const SceneDesc &S, const uint32
   return true;
 }
 
-struct CtaSync {
-  __device__ __forceinline__ void operator()() const { __syncthreads(); }
-};
-struct WarpSync {
-  __device__ __forceinline__ void operator()() const { __syncwarp(); }
-};
+// One pass of a warp over the `total` sources of a cell's neighbourhood: the
+// sums of kB bodies per lane, kSplit lanes to a body (the same values in each
+// of them).  `self[b]` is the slot of body b, `slot` arguments index pos4.
+template <uint32_t kSplit, uint32_t kB>
+__device__ __forceinline__ void p2p_pass(P2PStage &T, P2PTerms &U, const float4 *__restrict__ pos4, uint32_t total,
+                                         float eps2, f32x2 mz, bool plain, const float (&px)[kB],
+                                         const float (&py)[kB], const float (&pz)[kB], const uint32_t (&self)[kB],
+                                         float3 (&out)[kB]) {
+  constexpr uint32_t kAll = 0xFFFFFFFFu, kNone = 0xFFFFFFFFu, kPer = kP2PChunk / 32u;
+  const uint32_t lane = threadIdx.x & 31u, sub = lane % kSplit;
+  P2PBody body[kB];
+  float3 acc[kB];
+#pragma unroll
+  for (uint32_t b = 0; b < kB; b++) {
+    body[b] = {pack2(-px[b], -px[b]), pack2(-py[b], -py[b]), pack2(-pz[b], -pz[b])};
+    acc[b] = make_float3(0.0f, 0.0f, 0.0f);
+  }
+  const f32x2 e2 = pack2(eps2, eps2);
+  uint32_t range[kPer];
+  float4 q[kPer];
+#pragma unroll
+  for (uint32_t i = 0; i < kPer; i++) range[i] = 0u;
+  auto fetch = [&](uint32_t base) {
+#pragma unroll
+    for (uint32_t i = 0; i < kPer; i++) {
+      const uint32_t v = base + 32u * i + lane;
+      q[i] = make_float4(kP2PFar, kP2PFar, kP2PFar, 0.0f);
+      if (v < total) {
+        while (v >= T.first[range[i] + 1u]) range[i]++;
+        q[i] = __ldg(&pos4[v + T.shift[range[i]]]);
+      }
+    }
+  };
+  fetch(0u);
+  for (uint32_t base = 0; base < total; base += kP2PChunk) {
+    bool near = plain;
+    __syncwarp();  // the previous chunk is consumed
+#pragma unroll
+    for (uint32_t i = 0; i < kPer; i++) {
+      T.x[32u * i + lane] = q[i].x;
+      T.y[32u * i + lane] = q[i].y;
+      T.z[32u * i + lane] = q[i].z;
+      near = near && fabsf(q[i].x) <= kP2PFar && fabsf(q[i].y) <= kP2PFar && fabsf(q[i].z) <= kP2PFar;
+    }
+    near = __all_sync(kAll, near);
+    __syncwarp();
+    if (base + kP2PChunk < total) fetch(base + kP2PChunk);
+    const uint32_t m = min(kP2PChunk, total - base);
+    if (!near) {
+      // Plain expressions; the first of a body's lanes sums for all.
+#pragma unroll
+      for (uint32_t b = 0; b < kB; b++) {
+        uint32_t at = kNone;  // the body's sequence index, if its slot is among these sources
+        for (uint32_t j = 0; j < 27u; j++) {
+          const uint32_t v = self[b] - T.shift[j];
+          const uint32_t end = j < 26u ? T.first[j + 1u] : total;
+          if (v >= T.first[j] && v < end) at = v;
+        }
+#ifdef RFMM_FAST_FLOAT
+        if (sub == 0u) acc[b] = p2p_chunk_checked(T, m, at - base, px[b], py[b], pz[b], eps2, acc[b]);
+#else
+        const uint32_t l0 = lane - sub;
+        float3 s = acc[b];
+        if (kSplit > 1u)
+          s = make_float3(__shfl_sync(kAll, acc[b].x, l0), __shfl_sync(kAll, acc[b].x, l0 + 1u),
+                          __shfl_sync(kAll, acc[b].x, l0 + 2u));
+        s = p2p_chunk_checked(T, m, at - base, px[b], py[b], pz[b], eps2, s);
+        if (kSplit > 1u) acc[b].x = sub == 0u ? s.x : (sub == 1u ? s.y : s.z);
+        else acc[b] = s;
+#endif
+      }
+      __syncwarp();
+      continue;
+    }
+#ifdef RFMM_FAST_FLOAT
+    // Fresh partial sums per chunk (the order of addition is free here).
+    f32x2 ax[kB], ay[kB], az[kB];
+#pragma unroll
+    for (uint32_t b = 0; b < kB; b++) ax[b] = ay[b] = az[b] = 0ull;
+#pragma unroll 2
+    for (uint32_t k = 0; k < m; k += 2u * kSplit) {
+      const f32x2 qx = *reinterpret_cast<const f32x2 *>(&T.x[k + 2u * sub]);
+      const f32x2 qy = *reinterpret_cast<const f32x2 *>(&T.y[k + 2u * sub]);
+      const f32x2 qz = *reinterpret_cast<const f32x2 *>(&T.z[k + 2u * sub]);
+#pragma unroll
+      for (uint32_t b = 0; b < kB; b++) p2p_two(qx, qy, qz, body[b], e2, mz, ax[b], ay[b], az[b]);
+    }
+#pragma unroll
+    for (uint32_t b = 0; b < kB; b++) {
+      float u, v;
+      unpack2(ax[b], u, v);
+      acc[b].x = acc[b].x + (u + v);
+      unpack2(ay[b], u, v);
+      acc[b].y = acc[b].y + (u + v);
+      unpack2(az[b], u, v);
+      acc[b].z = acc[b].z + (u + v);
+    }
+#else
+    if constexpr (kSplit == 1u) {
+#pragma unroll 2
+      for (uint32_t k = 0; k < m; k += 4u) {
+        const ulonglong2 qx = *reinterpret_cast<const ulonglong2 *>(&T.x[k]);
+        const ulonglong2 qy = *reinterpret_cast<const ulonglong2 *>(&T.y[k]);
+        const ulonglong2 qz = *reinterpret_cast<const ulonglong2 *>(&T.z[k]);
+        f32x2 tx, ty, tz, ux, uy, uz;
+        p2p_two(qx.x, qy.x, qz.x, body[0], e2, mz, tx, ty, tz);
+        p2p_two(qx.y, qy.y, qz.y, body[0], e2, mz, ux, uy, uz);
+        acc[0].x = add_both(add_both(acc[0].x, tx), ux);
+        acc[0].y = add_both(add_both(acc[0].y, ty), uy);
+        acc[0].z = add_both(add_both(acc[0].z, tz), uz);
+      }
+    } else {
+      // A group of 4 kSplit sources, four to a lane; acc[0].x is the running
+      // sum of component `sub` (lanes 3 and up of a body: unused).
+      constexpr uint32_t kGroup = 4u * kSplit, kRow = kSplit == 4u ? kP2PTermComp : kGroup;
+      const uint32_t row0 = (lane / kSplit) * kP2PTermBody;
+      const uint32_t put = row0 + 4u * sub, get = row0 + min(sub, 2u) * kRow;
+      auto eval = [&](uint32_t k, ulonglong2 &tx, ulonglong2 &ty, ulonglong2 &tz) {
+        const ulonglong2 qx = *reinterpret_cast<const ulonglong2 *>(&T.x[k + 4u * sub]);
+        const ulonglong2 qy = *reinterpret_cast<const ulonglong2 *>(&T.y[k + 4u * sub]);
+        const ulonglong2 qz = *reinterpret_cast<const ulonglong2 *>(&T.z[k + 4u * sub]);
+        p2p_two(qx.x, qy.x, qz.x, body[0], e2, mz, tx.x, ty.x, tz.x);
+        p2p_two(qx.y, qy.y, qz.y, body[0], e2, mz, tx.y, ty.y, tz.y);
+      };
+      auto store = [&](float *buf, ulonglong2 tx, ulonglong2 ty, ulonglong2 tz) {
+        *reinterpret_cast<ulonglong2 *>(buf + put) = tx;
+        *reinterpret_cast<ulonglong2 *>(buf + put + kRow) = ty;
+        *reinterpret_cast<ulonglong2 *>(buf + put + 2u * kRow) = tz;
+        __syncwarp();
+      };
+      auto add4 = [&](const float *at) {
+        const float4 t = *reinterpret_cast<const float4 *>(at);
+        acc[0].x = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(acc[0].x, t.x), t.y), t.z), t.w);
+      };
+      ulonglong2 tx, ty, tz;
+      eval(0u, tx, ty, tz);
+      store(U.v[0], tx, ty, tz);
+      if constexpr (kSplit == 4u) {
+        // The next group's terms are evaluated while this one's are added;
+        // each buffer is read before the barrier that precedes its next store.
+#pragma unroll 2
+        for (uint32_t k = 0; k < m; k += kGroup) {
+          const float *buf = U.v[(k / kGroup) & 1u] + get;
+          const bool more = k + kGroup < m;
+          if (more) eval(k + kGroup, tx, ty, tz);
+#pragma unroll
+          for (uint32_t i = 0; i < kGroup; i += 4u) add4(buf + i);
+          if (more) store(U.v[(k / kGroup + 1u) & 1u], tx, ty, tz);
+        }
+        __syncwarp();
+      } else {
+#pragma unroll 8
+        for (uint32_t i = 0; i < m; i += 4u) add4(U.v[0] + get + i);
+        __syncwarp();
+      }
+    }
+#endif
+  }
+#pragma unroll
+  for (uint32_t b = 0; b < kB; b++) {
+    if constexpr (kSplit > 1u) {
+#ifdef RFMM_FAST_FLOAT
+#pragma unroll
+      for (uint32_t o = 1u; o < kSplit; o <<= 1) {
+        acc[b].x = acc[b].x + __shfl_xor_sync(kAll, acc[b].x, o);
+        acc[b].y = acc[b].y + __shfl_xor_sync(kAll, acc[b].y, o);
+        acc[b].z = acc[b].z + __shfl_xor_sync(kAll, acc[b].z, o);
+      }
+#else
+      const uint32_t l0 = lane - sub;
+      const float c = acc[b].x;
+      acc[b] = make_float3(__shfl_sync(kAll, c, l0), __shfl_sync(kAll, c, l0 + 1u), __shfl_sync(kAll, c, l0 + 2u));
+#endif
+    }
+    out[b] = acc[b];
+  }
+}
 
-__global__ void __launch_bounds__(256, 4) k_near_p2p(const SceneDesc *__restrict__ scenes,
+template <uint32_t kSplit>
+__global__ void __launch_bounds__(32 * kP2PWarps, 4) k_near_p2p(const SceneDesc *__restrict__ scenes,
                                                   const uint32_t *__restrict__ tile_scene,
                                                   const float4 *__restrict__ pos4,
                                                   const uint32_t *__restrict__ starts,
@@ -536,94 +809,148 @@ __global__ void __launch_bounds__(256, 4) k_near_p2p(const SceneDesc *__restrict
                                                   uint32_t tiles,
                                                   const uint32_t *__restrict__ tile_list,
                                                   Counters *__restrict__ ctr,
-                                                  float4 *__restrict__ near_out,
+                                                  float4 *__restrict__ near_out, float minus_zero,
                                                   unsigned long long *__restrict__ stamp) {
-  __shared__ float4 buf[kTile];
-  __shared__ SceneDesc S;
-  __shared__ uint32_t s_cell[5];  // tid 0's sample cell: key, level, x, y, z
-  __shared__ uint32_t s_next;
-  const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+  constexpr uint32_t kUnit = kP2PUnit<kSplit>, kUnitsPerTile = kTile / kUnit, kBody = 32u / kSplit;
+  static_assert(kTile % kUnit == 0u, "a unit never crosses a tile");
+  constexpr uint32_t kAll = 0xFFFFFFFFu, kNone = 0xFFFFFFFFu;
+  __shared__ P2PStage stage[kP2PWarps];
+  __shared__ P2PTerms terms[kP2PBodies == 1u ? kP2PWarps : 1u];  // the fast variant has no use for it
+  const uint32_t lane = threadIdx.x & 31u, sub = lane % kSplit;
+  P2PStage &T = stage[threadIdx.x >> 5];
+  P2PTerms &U = terms[kP2PBodies == 1u ? threadIdx.x >> 5 : 0u];
+  const f32x2 mz = pack2(minus_zero, minus_zero);
   grid_dependency_wait();  // the upward pass resolved this step's sample cells
   stamp_begin(stamp);
   const uint32_t ntiles = tile_list != nullptr ? min(ctr->tiles_active, tiles) : tiles;
-  // Tiles are taken one at a time from a counter (reset by this step's
-  // upward pass): a tile's cost is its bodies times the sources around their
-  // sample cell, which spans two orders of magnitude between sparse and
-  // core leaves, so a static share leaves most SMs idle behind the heaviest.
-  auto grab = [&]() -> uint32_t {
-    __syncthreads();
-    if (tid == 0) s_next = atomicAdd(&ctr->p2p_cursor, 1u);
-    __syncthreads();
-    return s_next;
-  };
-  uint32_t cur = 0xFFFFFFFFu;
-  for (uint32_t i = grab(); i < ntiles; i = grab()) {
-    const uint32_t tile = tile_list != nullptr ? tile_list[i] : i;
-    const uint32_t sc = tile_scene[tile];
-    if (sc != cur) {
-      load_scene(S, scenes, sc);  // barriers inside: the previous tile's buffer is free
-      cur = sc;
-    } else {
-      __syncthreads();
-    }
-    const uint32_t slot = tile * kTile + tid;
-    const bool active = slot - S.body_off < S.n;
-    float px = 0.0f, py = 0.0f, pz = 0.0f;
-    uint32_t level = 0u, lx = 0u, ly = 0u, lz = 0u, key = 0xFFFFFFFFu;
-    if (active) {
-      const float4 p = pos4[slot];
-      px = p.x;
-      py = p.y;
-      pz = p.z;
-      key = sample_cell(S, px, py, pz, mom, choice, level, lx, ly, lz);
-    }
-    const uint32_t csh = S.depth - level;
-    if (tid == 0) {  // slot 0 of a tile always holds a body
-      s_cell[0] = key;
-      s_cell[1] = level;
-      s_cell[2] = lx >> csh;
-      s_cell[3] = ly >> csh;
-      s_cell[4] = lz >> csh;
-    }
-    __syncthreads();
+  const uint32_t nunits = ntiles * kUnitsPerTile;
+  for (;;) {
+    // A unit's cost is its bodies times the sources around their sample
+    // cells, two orders of magnitude apart between sparse and core leaves:
+    // units come from a counter (reset by this step's upward pass).
+    uint32_t unit = 0u;
+    if (lane == 0u) unit = atomicAdd(&ctr->p2p_cursor, 1u);
+    unit = __shfl_sync(kAll, unit, 0);
+    if (unit >= nunits) break;
+    const uint32_t entry = unit / kUnitsPerTile;
+    const uint32_t tile = tile_list != nullptr ? tile_list[entry] : entry;
+    const SceneDesc &S = scenes[tile_scene[tile]];
+    const uint32_t slot0 = tile * kTile + (unit % kUnitsPerTile) * kUnit + lane / kSplit;
     const float eps2 = S.softening * S.softening;
-    float sx = 0.0f, sy = 0.0f, sz = 0.0f;
-    const bool tile_uniform = __syncthreads_and(!active || key == s_cell[0]) != 0;
-    if (tile_uniform) {
-      // Every thread takes the same branches: tid 0's cell drives the loops.
-      for (uint32_t j = 0; j < 27u; j++) {
-        uint32_t lo, hi;
-        if (neighbour_range(S, starts, s_cell[1], s_cell[2], s_cell[3], s_cell[4], j, lo, hi))
-          p2p_staged_range<kTile>(pos4, lo, hi, buf, tid, slot, px, py, pz, eps2, sx, sy, sz,
-                                  CtaSync());
+
+    float px[kP2PBodies], py[kP2PBodies], pz[kP2PBodies];
+    uint32_t level[kP2PBodies], cx[kP2PBodies], cy[kP2PBodies], cz[kP2PBodies], key[kP2PBodies], self[kP2PBodies];
+    float3 sum[kP2PBodies];
+    bool plain = eps2 >= 0x1p-80f && eps2 <= 0x1p120f;
+#pragma unroll
+    for (uint32_t b = 0; b < kP2PBodies; b++) {
+      const uint32_t slot = slot0 + kBody * b;
+      self[b] = slot;
+      px[b] = py[b] = pz[b] = 0.0f;
+      level[b] = cx[b] = cy[b] = cz[b] = 0u;
+      key[b] = kNone;
+      if (slot - S.body_off < S.n) {
+        const float4 p = pos4[slot];
+        px[b] = p.x;
+        py[b] = p.y;
+        pz[b] = p.z;
+        key[b] = sample_cell(S, p.x, p.y, p.z, mom, choice, level[b], cx[b], cy[b], cz[b]);
+        const uint32_t csh = S.depth - level[b];
+        cx[b] >>= csh;
+        cy[b] >>= csh;
+        cz[b] >>= csh;
       }
-    } else {
-      // Warps whose active bodies share a cell stage their own 32-source slice.
-      const uint32_t amask = __ballot_sync(0xFFFFFFFFu, active);
-      const uint32_t lead = amask != 0u ? (uint32_t)__ffs(amask) - 1u : 0u;
-      const uint32_t wkey = __shfl_sync(0xFFFFFFFFu, key, lead);
-      const bool warp_uniform = __all_sync(0xFFFFFFFFu, !active || key == wkey);
-      if (amask == 0u) {
-        // Padding only: nothing to sum.
-      } else if (warp_uniform) {
-        const uint32_t wl = __shfl_sync(0xFFFFFFFFu, level, lead);
-        const uint32_t wx = __shfl_sync(0xFFFFFFFFu, lx >> csh, lead);
-        const uint32_t wy = __shfl_sync(0xFFFFFFFFu, ly >> csh, lead);
-        const uint32_t wz = __shfl_sync(0xFFFFFFFFu, lz >> csh, lead);
-        float4 *wbuf = buf + 32u * warp;
-        for (uint32_t j = 0; j < 27u; j++) {
-          uint32_t lo, hi;
-          if (neighbour_range(S, starts, wl, wx, wy, wz, j, lo, hi))
-            p2p_staged_range<32u>(pos4, lo, hi, wbuf, lane, slot, px, py, pz, eps2, sx, sy, sz,
-                                  WarpSync());
-        }
-      } else if (active) {
-        const P2PView V{pos4, starts, slot};
-        float sp;
-        p2p_sums<false>(S, V, level, lx >> csh, ly >> csh, lz >> csh, px, py, pz, sx, sy, sz, sp);
-      }
+      plain = plain && fabsf(px[b]) < 0.5f * kP2PFar && fabsf(py[b]) < 0.5f * kP2PFar &&
+              fabsf(pz[b]) < 0.5f * kP2PFar;
+      sum[b] = make_float3(0.0f, 0.0f, 0.0f);
     }
-    if (active) near_out[slot] = make_float4(sx, sy, sz, 0.0f);
+    plain = __all_sync(kAll, plain);
+
+    // One sample cell after the other.
+    bool done[kP2PBodies];
+#pragma unroll
+    for (uint32_t b = 0; b < kP2PBodies; b++) done[b] = key[b] == kNone;
+    for (;;) {
+      uint32_t gkey = kNone, gl = 0u, gx = 0u, gy = 0u, gz = 0u;
+#pragma unroll
+      for (uint32_t b = 0; b < kP2PBodies; b++) {
+        const uint32_t open = __ballot_sync(kAll, !done[b]);
+        if (gkey == kNone && open != 0u) {
+          const uint32_t lead = (uint32_t)__ffs(open) - 1u;
+          gkey = __shfl_sync(kAll, key[b], lead);
+          gl = __shfl_sync(kAll, level[b], lead);
+          gx = __shfl_sync(kAll, cx[b], lead);
+          gy = __shfl_sync(kAll, cy[b], lead);
+          gz = __shfl_sync(kAll, cz[b], lead);
+        }
+      }
+      if (gkey == kNone) break;
+      // The neighbour ranges as one sequence of `total` sources.
+      uint32_t lo = 0u, hi = 0u;
+      if (lane < 27u && !neighbour_range(S, starts, gl, gx, gy, gz, lane, lo, hi)) lo = hi = 0u;
+      uint32_t upto = hi - lo;
+#pragma unroll
+      for (uint32_t off = 1u; off < 32u; off <<= 1) {
+        const uint32_t t = __shfl_up_sync(kAll, upto, off);
+        if (lane >= off) upto += t;
+      }
+      const uint32_t total = __shfl_sync(kAll, upto, 31);
+      __syncwarp();  // the previous cell's ranges and chunk are consumed
+      if (lane < 27u) {
+        T.first[lane] = upto - (hi - lo);
+        T.shift[lane] = lo - (upto - (hi - lo));
+      }
+      if (lane == 27u) T.first[27] = kNone;
+      __syncwarp();
+
+      // The unit's bodies in this cell (a body's first lane counts for it).
+      uint32_t members[kP2PBodies], count = 0u;
+#pragma unroll
+      for (uint32_t b = 0; b < kP2PBodies; b++) {
+        members[b] = __ballot_sync(kAll, key[b] == gkey && sub == 0u);
+        count += __popc(members[b]);
+      }
+      if (count == 1u) {
+#pragma unroll
+        for (uint32_t b = 0; b < kP2PBodies; b++) {
+          if (members[b] == 0u) continue;
+          const uint32_t owner = (uint32_t)__ffs(members[b]) - 1u;
+          const float ox[1] = {__shfl_sync(kAll, px[b], owner)}, oy[1] = {__shfl_sync(kAll, py[b], owner)},
+                      oz[1] = {__shfl_sync(kAll, pz[b], owner)};
+          const uint32_t oself[1] = {__shfl_sync(kAll, self[b], owner)};
+          float3 o[1];
+          p2p_pass<32u, 1u>(T, U, pos4, total, eps2, mz, plain, ox, oy, oz, oself, o);
+          if (lane / kSplit == owner / kSplit) sum[b] = o[0];
+        }
+      } else if (kSplit == 1u && count <= 8u) {
+        // Four lanes to a body: quad j takes the cell's j-th body.
+#pragma unroll
+        for (uint32_t b = 0; b < kP2PBodies; b++) {
+          if (members[b] == 0u) continue;
+          const uint32_t rank = __popc(members[b] & ((1u << lane) - 1u));
+          const uint32_t owner = __fns(members[b], 0u, (int)min(lane >> 2, (uint32_t)__popc(members[b]) - 1u) + 1);
+          const float ox[1] = {__shfl_sync(kAll, px[b], owner)}, oy[1] = {__shfl_sync(kAll, py[b], owner)},
+                      oz[1] = {__shfl_sync(kAll, pz[b], owner)};
+          const uint32_t oself[1] = {__shfl_sync(kAll, self[b], owner)};
+          float3 o[1];
+          p2p_pass<4u, 1u>(T, U, pos4, total, eps2, mz, plain, ox, oy, oz, oself, o);
+          const float rx = __shfl_sync(kAll, o[0].x, 4u * rank & 31u), ry = __shfl_sync(kAll, o[0].y, 4u * rank & 31u),
+                      rz = __shfl_sync(kAll, o[0].z, 4u * rank & 31u);
+          if (key[b] == gkey) sum[b] = make_float3(rx, ry, rz);
+        }
+      } else {
+        float3 o[kP2PBodies];
+        p2p_pass<kSplit, kP2PBodies>(T, U, pos4, total, eps2, mz, plain, px, py, pz, self, o);
+#pragma unroll
+        for (uint32_t b = 0; b < kP2PBodies; b++)
+          if (key[b] == gkey) sum[b] = o[b];
+      }
+#pragma unroll
+      for (uint32_t b = 0; b < kP2PBodies; b++) done[b] = done[b] || key[b] == gkey;
+    }
+#pragma unroll
+    for (uint32_t b = 0; b < kP2PBodies; b++)
+      if (key[b] != kNone && sub == 0u) near_out[slot0 + kBody * b] = make_float4(sum[b].x, sum[b].y, sum[b].z, 0.0f);
   }
   stamp_end(stamp);
   grid_dependents_may_launch();
@@ -1012,24 +1339,39 @@ void launch_integrate(const LaunchCtx &L, uint32_t tiles) {
                      (const float4 *)L.near4, stamp_rec(L, 3u));
 }
 
-// The P2P grid: one wave of this kernel's resident CTAs (its register
-// budget allows fewer per SM than integrate's), at most one per tile.
-static uint32_t near_p2p_grid(const LaunchCtx &L, uint32_t tiles) {
+// One wave of the pair-sum kernel's resident CTAs, at most one warp per unit.
+template <uint32_t kSplit>
+static void launch_near_p2p_split(const LaunchCtx &L, uint32_t tiles) {
   static const uint32_t per_sm = [] {
     int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_near_p2p, kTile, 0) != cudaSuccess || n < 1)
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_near_p2p<kSplit>, 32 * kP2PWarps, 0) != cudaSuccess ||
+        n < 1)
       n = 1;
     return (uint32_t)n;
   }();
-  const uint32_t grid = (L.sms ? L.sms : 1u) * per_sm;
-  return tiles < grid ? tiles : grid;
+  const uint32_t units = tiles * (kTile / kP2PUnit<kSplit>), wave = (L.sms ? L.sms : 1u) * per_sm;
+  const uint32_t ctas = (units + kP2PWarps - 1u) / kP2PWarps;
+  launch_step_kernel(L, k_near_p2p<kSplit>, dim3(ctas < wave ? ctas : wave), dim3(32u * kP2PWarps), 0, L.scenes,
+                     L.tile_scene, (const float4 *)L.pos4, (const uint32_t *)L.starts_out,
+                     (const uint4 *)L.mom, (const uint32_t *)L.choice, tiles, L.tile_list, L.ctr,
+                     L.near4, -0.0f, stamp_rec(L, 5u));
 }
 
 void launch_near_p2p(const LaunchCtx &L, uint32_t tiles) {
-  launch_step_kernel(L, k_near_p2p, dim3(near_p2p_grid(L, tiles)), dim3(kTile), 0, L.scenes,
-                     L.tile_scene, (const float4 *)L.pos4, (const uint32_t *)L.starts_out,
-                     (const uint4 *)L.mom, (const uint32_t *)L.choice, tiles, L.tile_list, L.ctr,
-                     L.near4, stamp_rec(L, 5u));
+  // Units of 8 bodies while units of 32 would leave warps idle: up to 8 per
+  // SM (38,912 slots on 152).  Exact, ms, 8 / 32: Plummer 16,384 0.55 / 0.68,
+  // 32,768 1.79 / 1.78, 120,001 9.6 / 8.8; uniform 16,384 0.13 / 0.18.  The
+  // fast variant's split costs nothing, so it always takes 16 (16 / 64:
+  // Plummer 16,384 0.33 / 0.76, 1,048,576 59.8 / 54.6, clusters 600,007
+  // 15.0 / 24.2).
+#ifdef RFMM_FAST_FLOAT
+  launch_near_p2p_split<4>(L, tiles);
+#else
+  if (tiles * (kTile / 32u) <= 8u * L.sms)
+    launch_near_p2p_split<4>(L, tiles);
+  else
+    launch_near_p2p_split<1>(L, tiles);
+#endif
 }
 
 void launch_deposit(const LaunchCtx &L, uint4 *moments, uint32_t tiles) {

@@ -128,3 +128,33 @@ def test_p2p_force_error_is_small(rfmm_mod, oracle_mod):
         s.set_near_mode(R.NEAR_P2P)
         p2p_rms, _ = s.force_error(2048, 3)
     assert p2p_rms < 0.05 and p2p_rms < 0.25 * ref_rms, (p2p_rms, ref_rms)
+
+
+def _same_or_nan(g, r, what):
+    """Bit equality where the oracle is a number; NaN where it is NaN."""
+    g, r = np.ascontiguousarray(g).view(np.float32).ravel(), np.ascontiguousarray(r).view(np.float32).ravel()
+    nan = np.isnan(r)
+    assert np.array_equal(np.isnan(g), nan), what
+    _same(g[~nan], r[~nan], what)
+
+
+@pytest.mark.parametrize("softening", [0.0, 1e-13, 1e-3])
+@pytest.mark.parametrize("n", [1, 31, 33, 65, 257, 1025, 40001])
+def test_p2p_unit_edges_and_unusual_bodies_bit_exact(rfmm_mod, oracle_mod, n, softening):
+    """Ragged units, no softening, coincident, distant and non-finite bodies."""
+    O, R = oracle_mod, rfmm_mod
+    from rfmm import scenes
+    p = scenes.make("plummer", n, 47)
+    if n > 60:
+        p["pos"][5] = p["pos"][6]
+        p["pos"][9] = [1e25, 0.0, 0.0]
+        p["pos"][11] = [-3e18, 2e18, 1.0]
+        p["pos"][17] = [np.inf, 0.1, 0.1]
+        p["pos"][23] = [np.nan, 0.2, 0.2]
+    st = O.OracleState(p, O.make_params(n, gravity=1.0, softening=softening, dt=5e-4, near_mode=1))
+    st.step(1)
+    with R.Solver(n, R.default_params(gravity=1.0, softening=softening, dt=5e-4)) as s:
+        s.set_near_mode(R.NEAR_P2P)
+        s.upload(p)
+        s.step(1)
+        _same_or_nan(s.particles(), st.particles, "particles")
