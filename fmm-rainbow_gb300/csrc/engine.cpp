@@ -174,13 +174,17 @@ int Engine::create(const std::vector<SceneSpec> &specs, Engine **out) {
   E->tiles_ = body_off / kTile;
   E->cells_ = cell_off;
   E->tasks_ = task_off;
-  // Sort key = scene rank above a Morton code of fine cells (level F >= depth,
-  // at most 8: one scene sorts in three 8-bit radix passes): bodies of one
-  // leaf stay contiguous and a warp's bodies stay spatially compact, so a few
-  // steps of drift still leave few leaf runs per warp.
+  // Sort key = scene rank above a Morton code of fine cells (level F >= the
+  // deepest tree's, at most 8): bodies of one leaf stay contiguous and a
+  // warp's bodies stay spatially compact, so a few steps of drift still leave
+  // few leaf runs per warp.  F is the finest level that takes no more 8-bit
+  // sort passes than the deepest leaf level does.
   {
     const uint32_t scene_bits = log2_ceil((uint32_t)specs.size());
-    const uint32_t fine = std::min(8u, (32u - scene_bits) / 3u);
+    uint32_t deepest = 0u;
+    for (const SceneDesc &d : E->scenes_) deepest = std::max(deepest, d.max_depth);
+    const uint32_t bits = std::min(32u, (scene_bits + 3u * deepest + 7u) / 8u * 8u);
+    const uint32_t fine = std::min(8u, (bits - scene_bits) / 3u);
     for (uint32_t i = 0; i < E->scenes_.size(); i++) {
       E->scenes_[i].key_level = fine;
       E->scenes_[i].key_base = scene_bits ? (i << (3u * fine)) : 0u;
@@ -216,8 +220,9 @@ int Engine::create(const std::vector<SceneSpec> &specs, Engine **out) {
   A((void **)&E->d_ctr_, sizeof(Counters));
   A((void **)&E->d_tickets_, 4 * kTicketStride * specs.size());
   A((void **)&E->d_tmaps_, sizeof(CUtensorMap) * 8 * specs.size());
-  A((void **)&E->sort_.hist, 4 * 256 * (size_t)sort_tiles(E->slots_));
-  A((void **)&E->sort_.totals, 4 * 256);
+  A((void **)&E->sort_.totals, 4 * 4 * 256);
+  A((void **)&E->sort_.status, 8 * sort_status_words(E->slots_));
+  A((void **)&E->sort_.state, sizeof(SortState));
   for (const SceneDesc &d : E->scenes_) E->max_depth_ = std::max(E->max_depth_, d.max_depth);
   A((void **)&E->d_starts_, 4 * C);
   A((void **)&E->d_leaf_blocks_, 4 * (size_t)leaf_sort_blocks(E->max_depth_) * specs.size());
@@ -289,6 +294,10 @@ int Engine::create(const std::vector<SceneSpec> &specs, Engine **out) {
   if (e == cudaSuccess) e = cudaMemsetAsync(E->d_lfield_, 0, 48 * C, E->stream_);
   if (e == cudaSuccess) e = cudaMemsetAsync(E->d_fields_, 0, 48 * C, E->stream_);
   if (e == cudaSuccess) e = cudaMemsetAsync(E->d_ctr_, 0, sizeof(Counters), E->stream_);
+  if (e == cudaSuccess) e = cudaMemsetAsync(E->sort_.totals, 0, 4 * 4 * 256, E->stream_);
+  if (e == cudaSuccess)  // no word of a fresh array may carry the first pass's tag
+    e = cudaMemsetAsync(E->sort_.status, 0, 8 * sort_status_words(E->slots_), E->stream_);
+  if (e == cudaSuccess) e = cudaMemsetAsync(E->sort_.state, 0, sizeof(SortState), E->stream_);
   if (e == cudaSuccess)
     e = cudaMemsetAsync(E->d_tickets_, 0, 4 * kTicketStride * specs.size(), E->stream_);
   if (e != cudaSuccess) {
@@ -656,7 +665,7 @@ int Engine::seed_galaxy(uint32_t scene) {
   return RFMM_OK;
 }
 
-uint32_t Engine::radix_sort_kernels() const { return 2u + 3u * ((key_bits_ + 7u) / 8u); }
+uint32_t Engine::radix_sort_kernels() const { return 2u + (key_bits_ + 7u) / 8u; }
 
 void Engine::enqueue_resort(uint32_t ppar, uint32_t count_par, unsigned long long *stamps) {
   // Leaf counting sort from the deposit of the current positions; `stamps`
@@ -856,8 +865,8 @@ int Engine::activate_many(const std::vector<Admission> &admissions) {
   // cleared trees, one gather with the leaf deposit into the current buffer.
   LaunchCtx L = ctx(mcur_, lpar_, scr);
   L.stream = as;
-  launch_keys(L, sort_.keys[0], sort_.vals[0], d_ids_[scr], 1, total, 0u, nullptr, admit_map_.dev);
-  const int r = radix_sort(as, sort_, total * kTile, key_bits_);
+  launch_keys(L, sort_, key_bits_, d_ids_[scr], 1, total, nullptr, admit_map_.dev);
+  const int r = radix_sort(L, sort_, total * kTile, key_bits_, admit_map_.dev);
   launch_clear_scenes(L, (uint32_t)scenes_.size(), which, d_mom_[mcur_], d_mom_[mcur_ ^ 1u], d_src_, d_aux_);
   launch_gather(L, sort_.vals[r], d_part_[scr], d_ids_[scr], d_part_[cur], d_ids_[cur], d_mom_[mcur_],
                 total, 0u, nullptr, admit_map_.dev);
@@ -867,7 +876,7 @@ int Engine::activate_many(const std::vector<Admission> &admissions) {
     RF_CK(cudaStreamWaitEvent(stream_, admit_ev_, 0));
   }
   for (uint32_t sc : slots) uploaded_[sc] = true;
-  launches_ += 3u + 3u * ((key_bits_ + 7u) / 8u);
+  launches_ += 3u + (key_bits_ + 7u) / 8u;
   committed_ = true;
   return RFMM_OK;
 }
@@ -903,18 +912,16 @@ int Engine::commit() {
     if (!u) return RFMM_ERR_STATE;
   LaunchCtx L = ctx(mcur_, lpar_, pcur_);
   // The key pass also numbers the bodies of scenes uploaded since the last
-  // commit in caller order.
-  launch_keys(L, sort_.keys[0], sort_.vals[0], d_ids_[pcur_], any_fresh_ ? 2 : 0, tiles_, 0u,
-              &fresh_);
+  // commit in caller order, and clears the moment, source and record buffers
+  // that the rebuilt tree starts from (the upward pass skips subtrees that are
+  // empty in both moment buffers).
+  const ClearTree clear{{d_mom_[mcur_], d_mom_[mcur_ ^ 1u], reinterpret_cast<uint4 *>(d_src_),
+                         reinterpret_cast<uint4 *>(d_aux_)},
+                        cells_};
+  launch_keys(L, sort_, key_bits_, d_ids_[pcur_], any_fresh_ ? 2 : 0, tiles_, &fresh_, nullptr, &clear);
   fresh_ = SceneMask{};
   any_fresh_ = false;
-  const int r = radix_sort(stream_, sort_, slots_, key_bits_);
-  // The rebuilt tree starts from cleared moment, source and record buffers
-  // (the upward pass skips subtrees that are empty in both moment buffers).
-  RF_CK(cudaMemsetAsync(d_mom_[mcur_], 0, 16ull * cells_, stream_));
-  RF_CK(cudaMemsetAsync(d_mom_[mcur_ ^ 1u], 0, 16ull * cells_, stream_));
-  RF_CK(cudaMemsetAsync(d_src_, 0, 16ull * cells_, stream_));
-  RF_CK(cudaMemsetAsync(d_aux_, 0, 16ull * cells_, stream_));
+  const int r = radix_sort(L, sort_, slots_, key_bits_);
   launch_gather(L, sort_.vals[r], d_part_[pcur_], d_ids_[pcur_], d_part_[pcur_ ^ 1u],
                 d_ids_[pcur_ ^ 1u], d_mom_[mcur_], tiles_, 0u, d_pos4_);
   launches_ += radix_sort_kernels();
@@ -948,8 +955,8 @@ void Engine::enqueue_p2p_sort(uint32_t mpar, uint32_t lpar, uint32_t ppar, uint4
   LaunchCtx L = ctx(mpar, lpar, ppar);
   launch_unpermute(L, d_ids_[ppar], d_part_[ppar ^ 1u], 0u, tiles_);
   LaunchCtx C = ctx(mpar, lpar, ppar ^ 1u);
-  launch_keys(C, sort_.keys[0], sort_.vals[0], d_ids_[ppar ^ 1u], 1, tiles_, 0u);
-  const int r = radix_sort(stream_, sort_, slots_, key_bits_);
+  launch_keys(C, sort_, key_bits_, d_ids_[ppar ^ 1u], 1, tiles_);
+  const int r = radix_sort(C, sort_, slots_, key_bits_);
   launch_gather(L, sort_.vals[r], d_part_[ppar ^ 1u], d_ids_[ppar ^ 1u], d_part_[ppar],
                 d_ids_[ppar], mom_into, tiles_, 0u, d_pos4_);
   launch_leaf_starts(L, sort_.keys[r], (uint32_t)scenes_.size());
@@ -1103,7 +1110,7 @@ int Engine::step(uint32_t steps) {
 int Engine::check_device_error() {
   RF_CK(cudaMemcpyAsync(h_ctr_, d_ctr_, sizeof(Counters), cudaMemcpyDeviceToHost, stream_));
   RF_CK(cudaStreamSynchronize(stream_));
-  if (h_ctr_->error == kDevErrTmaTimeout) return RFMM_ERR_TIMEOUT;
+  if (h_ctr_->error == kDevErrTmaTimeout || h_ctr_->error == kDevErrSortTimeout) return RFMM_ERR_TIMEOUT;
   if (h_ctr_->error != 0u) return RFMM_ERR_DEVICE;
   return RFMM_OK;
 }

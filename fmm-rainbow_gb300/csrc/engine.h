@@ -166,7 +166,7 @@ class Engine {
   // kNearP2P end of step: bodies back to caller order, leaf-key sort, gather
   // with the deposit into `mom_into`, position snapshot and leaf starts.
   void enqueue_p2p_sort(uint32_t mpar, uint32_t lpar, uint32_t ppar, uint4 *mom_into);
-  uint32_t p2p_sort_kernels() const { return 4u + 3u * ((key_bits_ + 7u) / 8u); }
+  uint32_t p2p_sort_kernels() const { return 4u + (key_bits_ + 7u) / 8u; }
   uint32_t near_mode_ = kNearReference;
   uint32_t float_mode_ = RFMM_FLOAT_EXACT;
   const StepLaunchers &K() const;

@@ -1083,40 +1083,55 @@ void launch_accel(const LaunchCtx &L, const uint32_t *ids, float4 *out, uint32_t
                                          L.choice, L.fields, out, tile_base, L.pos4, L.starts_out);
 }
 
+// Sort keys of the bodies, a tile at a time, and the totals of the keys'
+// 8-bit digits for the sort's passes (counted per CTA in shared memory, one
+// global addition per CTA and digit).  The grid also clears the tree buffers
+// that the deposit after the sort starts from, so no separate fills run.
 __global__ void __launch_bounds__(256) k_keys(const SceneDesc *__restrict__ scenes,
                                               const uint32_t *__restrict__ tile_scene,
                                               const float4 *__restrict__ part,
-                                              uint32_t *__restrict__ keys, uint32_t *__restrict__ vals,
-                                              uint32_t *__restrict__ ids, int fresh_ids,
-                                              uint32_t tile_base,
+                                              uint32_t *__restrict__ keys, uint32_t *__restrict__ ids,
+                                              int fresh_ids, uint32_t tiles,
                                               const __grid_constant__ SceneMask fresh,
-                                              const uint32_t *__restrict__ tile_map) {
-  const uint32_t tile = tile_map != nullptr ? tile_map[blockIdx.x] : tile_base + blockIdx.x;
-  const uint32_t sc = tile_scene[tile];
-  const SceneDesc &S = scenes[sc];
-  const uint32_t slot = tile * kTile + threadIdx.x;
-  const uint32_t out = blockIdx.x * kTile + threadIdx.x;  // keys/vals are relative to tile_base
-  const uint32_t local = slot - S.body_off;
-  const uint32_t F = S.key_level;
-  uint32_t key = S.key_base | ((1u << (3u * F)) - 1u);  // padding sorts after its scene's bodies
-  if (local < S.n && S.near_mode == kNearP2P) {
-    // Leaf key only: bodies of a leaf keep their input (caller) order.
-    const float4 p = part[2u * slot];
-    const uint32_t dim = 1u << S.depth;
-    key = S.key_base | (morton3(cell_of_unit(unit_coord(p.x), dim), cell_of_unit(unit_coord(p.y), dim),
-                                cell_of_unit(unit_coord(p.z), dim))
-                        << (3u * (F - S.depth)));
-  } else if (local < S.n) {
-    const float4 p = part[2u * slot];
-    const uint32_t dim = 1u << F;
-    // floor(u * 2^F) >> (F - depth) == floor(u * 2^depth): the fine key refines the leaf key.
-    key = S.key_base | (spread3(cell_of_unit(unit_coord(p.x), dim)) |
-                        (spread3(cell_of_unit(unit_coord(p.y), dim)) << 1) |
-                        (spread3(cell_of_unit(unit_coord(p.z), dim)) << 2));
+                                              const uint32_t *__restrict__ tile_map, uint32_t digits,
+                                              uint32_t *__restrict__ totals, const ClearTree clear) {
+  __shared__ uint32_t s_total[4][256];
+#pragma unroll
+  for (uint32_t d = 0; d < 4u; d++) s_total[d][threadIdx.x] = 0u;
+  grid_dependency_wait();
+  __syncthreads();
+  for (uint32_t i = blockIdx.x; i < tiles; i += gridDim.x) {
+    const uint32_t tile = tile_map != nullptr ? tile_map[i] : i;
+    const uint32_t sc = tile_scene[tile];
+    const SceneDesc &S = scenes[sc];
+    const uint32_t slot = tile * kTile + threadIdx.x;
+    const uint32_t local = slot - S.body_off;
+    const uint32_t F = S.key_level;
+    uint32_t key = S.key_base | ((1u << (3u * F)) - 1u);  // padding sorts after its scene's bodies
+    if (local < S.n) {
+      // The key cell: in kNearP2P the leaf only (bodies of a leaf keep their
+      // input, caller, order), else a fine cell; floor(u * 2^F) >> (F - depth)
+      // == floor(u * 2^depth), so the fine key refines the leaf key.
+      const float4 p = part[2u * slot];
+      const uint32_t level = S.near_mode == kNearP2P ? S.depth : F, dim = 1u << level;
+      key = S.key_base | (morton3(cell_of_unit(unit_coord(p.x), dim), cell_of_unit(unit_coord(p.y), dim),
+                                  cell_of_unit(unit_coord(p.z), dim))
+                          << (3u * (F - level)));
+    }
+    keys[i * kTile + threadIdx.x] = key;
+    for (uint32_t d = 0; d < digits; d++) atomicAdd(&s_total[d][(key >> (8u * d)) & 255u], 1u);
+    if (fresh_ids == 1 || (fresh_ids == 2 && ((fresh.bits[sc >> 5] >> (sc & 31u)) & 1u))) ids[slot] = local;
   }
-  keys[out] = key;
-  vals[out] = slot;
-  if (fresh_ids == 1 || (fresh_ids == 2 && ((fresh.bits[sc >> 5] >> (sc & 31u)) & 1u))) ids[slot] = local;
+  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < clear.words; i += gridDim.x * blockDim.x) {
+#pragma unroll
+    for (uint32_t b = 0; b < 4u; b++) clear.buf[b][i] = zero;
+  }
+  __syncthreads();
+  for (uint32_t d = 0; d < digits; d++) {
+    const uint32_t c = s_total[d][threadIdx.x];
+    if (c != 0u) atomicAdd(&totals[256u * d + threadIdx.x], c);
+  }
 }
 
 // Apply a permutation to the resident bodies (and their caller ids).  With
@@ -1144,6 +1159,7 @@ __global__ void __launch_bounds__(256) k_gather(const SceneDesc *__restrict__ sc
     cta_tile_range(tiles, t0, t1);
     T.clear();
   }
+  grid_dependency_wait();  // the permutation is complete
   uint32_t cur = 0xFFFFFFFFu;
   for (uint32_t i = t0; i < t1; i++) {
     const uint32_t tile = tile_map != nullptr ? tile_map[i] : tile_base + i;
@@ -1379,20 +1395,21 @@ void launch_deposit(const LaunchCtx &L, uint4 *moments, uint32_t tiles) {
                                                          tiles, L.tile_list, L.ctr);
 }
 
-void launch_keys(const LaunchCtx &L, uint32_t *keys, uint32_t *vals, uint32_t *ids, int fresh_ids,
-                 uint32_t tiles, uint32_t tile_base, const SceneMask *fresh,
-                 const uint32_t *tile_map) {
+void launch_keys(const LaunchCtx &L, const SortScratch &s, uint32_t bits, uint32_t *ids, int fresh_ids,
+                 uint32_t tiles, const SceneMask *fresh, const uint32_t *tile_map, const ClearTree *clear) {
   static const SceneMask kNone{};
-  k_keys<<<tiles, kTile, 0, L.stream>>>(L.scenes, L.tile_scene, L.part, keys, vals, ids, fresh_ids,
-                                        tile_base, fresh != nullptr ? *fresh : kNone, tile_map);
+  const uint32_t wave = 8u * L.sms;
+  launch_step_kernel(L, k_keys, dim3(tiles < wave ? tiles : wave), dim3(kTile), 0, L.scenes, L.tile_scene,
+                     (const float4 *)L.part, s.keys[0], ids, fresh_ids, tiles, fresh != nullptr ? *fresh : kNone,
+                     tile_map, (bits + 7u) / 8u, s.totals, clear != nullptr ? *clear : ClearTree{});
 }
 
 void launch_gather(const LaunchCtx &L, const uint32_t *perm, const float4 *part_in,
                    const uint32_t *ids_in, float4 *part_out, uint32_t *ids_out, uint4 *deposit_into,
                    uint32_t tiles, uint32_t tile_base, float4 *pos_out, const uint32_t *tile_map) {
   const uint32_t grid = deposit_into != nullptr ? body_grid(L, tiles) : tiles;
-  k_gather<<<grid, kTile, 0, L.stream>>>(L.scenes, L.tile_scene, perm, part_in, ids_in, part_out,
-                                         ids_out, deposit_into, tiles, tile_base, pos_out, tile_map);
+  launch_step_kernel(L, k_gather, dim3(grid), dim3(kTile), 0, L.scenes, L.tile_scene, perm, part_in, ids_in,
+                     part_out, ids_out, deposit_into, tiles, tile_base, pos_out, tile_map);
 }
 
 // Per-leaf body ranges of the leaf-sorted scenes (kNearP2P): entry m of a

@@ -7,13 +7,20 @@
 // keys, and the deposit is a segmented reduction over those runs.  The sort
 // is stable, so the resident order is a deterministic function of the input.
 //
-// Per 8-bit pass:
-//   k_sort_hist     per 2048-key tile, digit histogram in shared memory
-//   k_sort_scan     one CTA per digit: exclusive scan of that digit's tile
-//                   counts (digit-major layout), plus the digit total
-//   k_sort_scatter  per tile: digit base + tile offset + stable rank inside
-//                   the tile (warp __match_any_sync ranks, warp prefix in
-//                   shared memory), then scatter
+// One launch per 8-bit pass (k_sort_pass).  The digit totals of every pass
+// come with the keys (k_keys counts them), so a tile only needs the counts of
+// the tiles before it: tiles are numbered by a ticket, publish their digit
+// counts and look back over their predecessors' (Merrill & Garland,
+// "Single-pass parallel prefix scan with decoupled look-back", 2016).  Ranks
+// inside a tile come from eight ballots per key and per-warp digit counters
+// (a match over 32 distinct digits takes about 230 cycles, the ballots about
+// 40), and a tile is put in digit order in shared memory before it is
+// written, so the stores run along digit runs.  What bounds a pass: memory
+// at millions of keys, latency (ticket, loads, ranks, look-back) below.
+// With histogram, scan and scatter launches per pass and separate fills of the
+// tree buffers before -> now, upload with sort and deposit, us: 4,096 bodies
+// 91 -> 18, 65,536 99 -> 25, 250,000 107 -> 43, 1,048,576 147 -> 104,
+// 5,242,880 539 -> 432.
 #include <cuda_runtime.h>
 
 #include "rfmm_device.cuh"
@@ -22,30 +29,25 @@
 namespace rfmm {
 
 constexpr uint32_t kSortThreads = 256u;
-constexpr uint32_t kSortItems = 8u;
-constexpr uint32_t kSortTile = kSortThreads * kSortItems;  // 2048 keys
+constexpr uint32_t kSortWarps = kSortThreads / 32u;
 
-uint32_t sort_tiles(uint32_t n) { return (n + kSortTile - 1u) / kSortTile; }
-
-__global__ void __launch_bounds__(kSortThreads) k_sort_hist(const uint32_t *__restrict__ keys,
-                                                            uint32_t n, uint32_t shift,
-                                                            uint32_t *__restrict__ hist,
-                                                            uint32_t ntiles) {
-  __shared__ uint32_t h[256];
-  const uint32_t tid = threadIdx.x, tile = blockIdx.x;
-  h[tid] = 0u;
-  __syncthreads();
-  for (uint32_t r = 0; r < kSortItems; r++) {
-    const uint32_t i = tile * kSortTile + r * kSortThreads + tid;
-    if (i < n) atomicAdd(&h[(keys[i] >> shift) & 255u], 1u);
-  }
-  __syncthreads();
-  hist[tid * ntiles + tile] = h[tid];
+// Keys per thread of a tile: many small tiles while they fit the GPU twice
+// over (latency), large ones beyond (fewer look-backs, longer digit runs;
+// 8 / 12 / 16 keys at 5,242,880 bodies: 479 / 453 / 438 us per upload).
+constexpr uint32_t kSortItemsSmall = 4u, kSortItemsLarge = 16u;
+constexpr uint32_t kSortSmallTiles = 304u;  // 2 per SM
+static uint32_t sort_tiles(uint32_t n) {
+  const uint32_t small = (n + kSortThreads * kSortItemsSmall - 1u) / (kSortThreads * kSortItemsSmall);
+  if (small <= kSortSmallTiles) return small;
+  return (n + kSortThreads * kSortItemsLarge - 1u) / (kSortThreads * kSortItemsLarge);
+}
+size_t sort_status_words(uint32_t capacity) {
+  const uint32_t t = sort_tiles(capacity);
+  return 256u * (size_t)(t < kSortSmallTiles ? kSortSmallTiles : t);  // smaller sorts may use more tiles
 }
 
 // Block-wide exclusive scan of one value per thread (256 threads).
-__device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t *warp_sums,
-                                                         uint32_t &total) {
+__device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t *warp_sums) {
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   uint32_t x = v;
 #pragma unroll
@@ -55,96 +57,199 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t *w
   }
   if (lane == 31u) warp_sums[warp] = x;
   __syncthreads();
-  if (warp == 0) {
-    uint32_t s = lane < (blockDim.x >> 5) ? warp_sums[lane] : 0u;
+  uint32_t before = 0u;
 #pragma unroll
-    for (uint32_t off = 1u; off < 32u; off <<= 1) {
-      const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, s, off);
-      if (lane >= off) s += y;
-    }
-    if (lane < (blockDim.x >> 5)) warp_sums[lane] = s;
-  }
-  __syncthreads();
-  const uint32_t before = warp == 0 ? 0u : warp_sums[warp - 1];
-  total = warp_sums[(blockDim.x >> 5) - 1];
+  for (uint32_t w = 0; w < kSortWarps; w++)
+    if (w < warp) before += warp_sums[w];
   __syncthreads();
   return before + x - v;
 }
 
-__global__ void __launch_bounds__(kSortThreads) k_sort_scan(uint32_t *__restrict__ hist,
-                                                            uint32_t ntiles,
-                                                            uint32_t *__restrict__ totals) {
-  __shared__ uint32_t warp_sums[32];
-  uint32_t *row = hist + blockIdx.x * ntiles;
-  uint32_t carry = 0u;
-  for (uint32_t base = 0; base < ntiles; base += kSortThreads) {
-    const uint32_t i = base + threadIdx.x;
-    const uint32_t v = i < ntiles ? row[i] : 0u;
-    uint32_t chunk_total;
-    const uint32_t ex = block_exclusive_scan(v, warp_sums, chunk_total);
-    if (i < ntiles) row[i] = carry + ex;
-    carry += chunk_total;
-  }
-  if (threadIdx.x == 0) totals[blockIdx.x] = carry;
+// A tile's published count of one digit: bits 0-31 the count, 32-33 what it
+// is, 34-63 the pass it belongs to (SortState::epoch, so words left by earlier
+// passes read as absent).
+constexpr uint32_t kSortOwn = 1u;   // the tile's own count
+constexpr uint32_t kSortUpTo = 2u;  // the count of every tile up to this one
+__device__ __forceinline__ unsigned long long sort_word(uint32_t epoch, uint32_t kind, uint32_t count) {
+  return ((unsigned long long)((epoch << 2) | kind) << 32) | count;
 }
 
-__global__ void __launch_bounds__(kSortThreads) k_sort_scatter(
+template <uint32_t kItems>
+__global__ void __launch_bounds__(kSortThreads) k_sort_pass(
     const uint32_t *__restrict__ keys_in, const uint32_t *__restrict__ vals_in,
-    uint32_t *__restrict__ keys_out, uint32_t *__restrict__ vals_out, uint32_t n, uint32_t shift,
-    const uint32_t *__restrict__ hist, const uint32_t *__restrict__ totals, uint32_t ntiles) {
-  __shared__ uint32_t base[256];
-  __shared__ uint32_t wcnt[kSortThreads / 32u][256];
-  __shared__ uint32_t warp_sums[32];
-  const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, tile = blockIdx.x;
-  {
-    uint32_t total;
-    const uint32_t digit_base = block_exclusive_scan(totals[tid], warp_sums, total);
-    base[tid] = digit_base + hist[tid * ntiles + tile];
+    const uint32_t *__restrict__ tile_map, uint32_t *__restrict__ keys_out, uint32_t *__restrict__ vals_out,
+    uint32_t n, uint32_t shift, uint32_t *__restrict__ totals, unsigned long long *__restrict__ status,
+    SortState *__restrict__ state, Counters *__restrict__ ctr) {
+  constexpr uint32_t kTileKeys = kSortThreads * kItems, kAll = 0xFFFFFFFFu;
+  __shared__ uint32_t s_key[kTileKeys], s_val[kTileKeys];
+  __shared__ uint32_t s_cnt[kSortWarps][256];  // per warp: digit counts, then first rank in the tile
+  __shared__ uint32_t s_out[256];              // per digit: output index minus index in the tile
+  __shared__ uint32_t s_sums[kSortWarps];
+  __shared__ uint32_t s_tile, s_epoch, s_stop;
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+#pragma unroll
+  for (uint32_t w = 0; w < kSortWarps; w++) s_cnt[w][tid] = 0u;
+  grid_dependency_wait();  // keys and totals, or the previous pass, are complete
+  if (tid == 0u) {
+    s_tile = atomicAdd(&state->ticket, 1u);
+    s_epoch = *reinterpret_cast<volatile uint32_t *>(&state->epoch);
+    s_stop = 0u;
   }
-  const uint32_t lt_mask = (1u << lane) - 1u;
-  for (uint32_t r = 0; r < kSortItems; r++) {
+  const uint32_t total = totals[tid];
+  __syncthreads();
+  const uint32_t tile = s_tile, epoch = s_epoch;
+  const uint32_t base = tile * kTileKeys + warp * 32u * kItems + lane;
+
+  // Warp w holds the tile's keys [32 kItems w, 32 kItems (w + 1)), 32 at a
+  // time: first the lanes with the same digit (independent ballots), then the
+  // ranks, one 32-key row after the other through the warp's counters.
+  uint32_t key[kItems], rank[kItems];
 #pragma unroll
-    for (uint32_t w = 0; w < kSortThreads / 32u; w++) wcnt[w][tid] = 0u;
-    __syncthreads();
-    const uint32_t i = tile * kSortTile + r * kSortThreads + tid;
-    const bool valid = i < n;
-    const uint32_t key = valid ? keys_in[i] : 0u;
-    const uint32_t digit = valid ? ((key >> shift) & 255u) : 256u + lane;
-    const uint32_t peers = __match_any_sync(0xFFFFFFFFu, digit);
-    const uint32_t rank = __popc(peers & lt_mask);
-    if (valid && rank == 0u) wcnt[warp][digit] = __popc(peers);
-    __syncthreads();
-    {
-      uint32_t run = base[tid];
+  for (uint32_t i = 0; i < kItems; i++) key[i] = base + 32u * i < n ? keys_in[base + 32u * i] : 0u;
 #pragma unroll
-      for (uint32_t w = 0; w < kSortThreads / 32u; w++) {
-        const uint32_t c = wcnt[w][tid];
-        wcnt[w][tid] = run;
-        run += c;
-      }
-      base[tid] = run;
+  for (uint32_t i = 0; i < kItems; i++) {
+    uint32_t peers = __ballot_sync(kAll, base + 32u * i < n);
+#pragma unroll
+    for (uint32_t b = 0; b < 8u; b++) {
+      const bool bit = (key[i] >> (shift + b)) & 1u;
+      const uint32_t ones = __ballot_sync(kAll, bit);
+      peers &= bit ? ones : ~ones;
     }
-    __syncthreads();
-    if (valid) {
-      const uint32_t pos = wcnt[warp][digit] + rank;
-      if (pos < n) {  // defensive: offsets from the histograms stay below n
-        keys_out[pos] = key;
-        vals_out[pos] = vals_in[i];
+    rank[i] = peers;
+  }
+#pragma unroll
+  for (uint32_t i = 0; i < kItems; i++) {
+    const uint32_t peers = rank[i], below = __popc(peers & ((1u << lane) - 1u));
+    const bool valid = base + 32u * i < n;
+    uint32_t *c = &s_cnt[warp][(key[i] >> shift) & 255u];
+    const uint32_t before = *c;
+    __syncwarp();
+    if (valid && below == 0u) *c = before + __popc(peers);
+    __syncwarp();
+    rank[i] = before + below;
+  }
+  __syncthreads();
+
+  // Values, needed after the look-back (first pass: a key's value is its slot).
+  uint32_t val[kItems];
+#pragma unroll
+  for (uint32_t i = 0; i < kItems; i++) {
+    const uint32_t at = base + 32u * i;
+    if (vals_in != nullptr) {
+      val[i] = at < n ? vals_in[at] : 0u;
+    } else {
+      val[i] = tile_map != nullptr && at < n ? tile_map[at / kTile] * kTile + at % kTile : at;
+    }
+  }
+
+  // Thread t: digit t.  Counts per warp become first ranks inside the tile.
+  uint32_t count = 0u;
+  {
+    uint32_t c[kSortWarps];
+#pragma unroll
+    for (uint32_t w = 0; w < kSortWarps; w++) {
+      c[w] = s_cnt[w][tid];
+      count += c[w];
+    }
+    volatile unsigned long long *mine = status + (size_t)tile * 256u + tid;
+    *mine = sort_word(epoch, tile == 0u ? kSortUpTo : kSortOwn, count);
+    const uint32_t first = block_exclusive_scan(count, s_sums);
+    uint32_t run = first;
+#pragma unroll
+    for (uint32_t w = 0; w < kSortWarps; w++) {
+      s_cnt[w][tid] = run;
+      run += c[w];
+    }
+    const uint32_t digit0 = block_exclusive_scan(total, s_sums);
+    // Look back until a tile that knows its whole prefix.  Tickets number
+    // tiles in the order their CTAs began, so every predecessor is running;
+    // the wait is bounded all the same.
+    uint32_t before = 0u;
+    if (tile != 0u) {
+      // Four predecessors per round trip, nearest first (1 / 4 / 8 / 16 at
+      // 1,048,576 bodies: 109 / 104 / 105 / 116 us per upload).
+      constexpr uint32_t kBack = 4u;
+      uint32_t back = tile;  // tiles [back, tile) are counted in `before`
+      bool open = true;
+      for (uint32_t polls = 0u; open;) {
+        unsigned long long w[kBack];
+#pragma unroll
+        for (uint32_t j = 0; j < kBack; j++)
+          w[j] = back > j ? *reinterpret_cast<volatile unsigned long long *>(status + (size_t)(back - 1u - j) * 256u + tid)
+                          : 0ull;
+        uint32_t used = 0u;
+#pragma unroll
+        for (uint32_t j = 0; j < kBack; j++) {
+          const uint32_t tag = (uint32_t)(w[j] >> 32);
+          if (open && used == j && (tag >> 2) == (epoch & 0x3FFFFFFFu) && (tag & 3u) != 0u) {
+            before += (uint32_t)w[j];
+            used = j + 1u;
+            open = (tag & 3u) != kSortUpTo;
+          }
+        }
+        back -= used;
+        if (open && used == 0u && ++polls == 1u << 22) {
+          if (atomicCAS(&ctr->error, 0u, (uint32_t)kDevErrSortTimeout) == 0u) ctr->error_info = tile;
+          s_stop = 1u;
+          break;
+        }
+      }
+      *mine = sort_word(epoch, kSortUpTo, before + count);
+    }
+    s_out[tid] = digit0 + before - first;
+  }
+  __syncthreads();
+
+  // Digit order in shared memory, then out along the digit runs.
+#pragma unroll
+  for (uint32_t i = 0; i < kItems; i++) {
+    const uint32_t from = base + 32u * i;
+    if (from < n) {
+      const uint32_t at = s_cnt[warp][(key[i] >> shift) & 255u] + rank[i];
+      s_key[at] = key[i];
+      s_val[at] = val[i];
+    }
+  }
+  __syncthreads();
+  if (s_stop == 0u) {
+    const uint32_t here = min(kTileKeys, n - tile * kTileKeys);
+#pragma unroll
+    for (uint32_t i = 0; i < kItems; i++) {
+      const uint32_t at = i * kSortThreads + tid;
+      if (at < here) {
+        const uint32_t k = s_key[at], out = s_out[(k >> shift) & 255u] + at;
+        if (out < n) {  // defensive: offsets from the counts stay below n
+          keys_out[out] = k;
+          vals_out[out] = s_val[at];
+        }
       }
     }
-    __syncthreads();
+  }
+  // The last CTA leaves the state ready for the next pass: this pass's
+  // totals cleared, a new epoch, tickets from zero.
+  if (tid == 0u) s_tile = atomicAdd(&state->done, 1u);
+  __syncthreads();
+  if (s_tile == gridDim.x - 1u) {
+    totals[tid] = 0u;
+    if (tid == 0u) {
+      state->ticket = 0u;
+      state->done = 0u;
+      state->epoch = epoch + 1u;
+    }
   }
 }
 
-int radix_sort(cudaStream_t stream, SortScratch &s, uint32_t n, uint32_t bits) {
+// Keys keys[0] (and their digit totals, s.totals) are in place; the values
+// start as the keys' slots (tile_map: as in launch_keys).
+int radix_sort(const LaunchCtx &L, SortScratch &s, uint32_t n, uint32_t bits, const uint32_t *tile_map) {
   const uint32_t ntiles = sort_tiles(n);
+  const auto pass = ntiles * kSortThreads * kSortItemsSmall >= n ? k_sort_pass<kSortItemsSmall>
+                                                                 : k_sort_pass<kSortItemsLarge>;
   int cur = 0;
   for (uint32_t shift = 0; shift < bits; shift += 8u) {
-    k_sort_hist<<<ntiles, kSortThreads, 0, stream>>>(s.keys[cur], n, shift, s.hist, ntiles);
-    k_sort_scan<<<256, kSortThreads, 0, stream>>>(s.hist, ntiles, s.totals);
-    k_sort_scatter<<<ntiles, kSortThreads, 0, stream>>>(s.keys[cur], s.vals[cur], s.keys[cur ^ 1],
-                                                        s.vals[cur ^ 1], n, shift, s.hist,
-                                                        s.totals, ntiles);
+    launch_step_kernel(L, pass, dim3(ntiles), dim3(kSortThreads), 0, (const uint32_t *)s.keys[cur],
+                       (const uint32_t *)(shift == 0u ? nullptr : s.vals[cur]), tile_map, s.keys[cur ^ 1],
+                       s.vals[cur ^ 1], n, shift, s.totals + 256u * (shift / 8u), s.status, s.state, L.ctr);
     cur ^= 1;
   }
   return cur;

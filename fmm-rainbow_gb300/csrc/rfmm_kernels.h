@@ -27,6 +27,16 @@ struct UploadSources {
   const float4 *p[kUploadChunk];
 };
 
+// Scratch of the radix sort (kernels_sort.cu).
+struct SortScratch {
+  uint32_t *keys[2];
+  uint32_t *vals[2];
+  uint32_t *totals;            // 4 x 256 digit totals: counted by launch_keys, cleared by the sort
+  unsigned long long *status;  // sort_status_words(capacity), zeroed once
+  SortState *state;            // zeroed once
+  uint32_t capacity;           // elements
+};
+
 // Device pointers one launch needs; filled by the engine for each step parity.
 struct LaunchCtx {
   cudaStream_t stream;
@@ -115,14 +125,18 @@ void launch_integrate(const LaunchCtx &L, uint32_t tiles);
 // kNearP2P: exact near-field pair sums of every body into L.near4.
 void launch_near_p2p(const LaunchCtx &L, uint32_t tiles);
 void launch_deposit(const LaunchCtx &L, uint4 *moments, uint32_t tiles);
-// keys/vals of tiles [tile_base, tile_base + tiles), written from index 0.
-// Body ids (caller order) are written too for every scene (fresh_ids 1) or
-// for the scenes set in *fresh (fresh_ids 2).
-// With `tile_map` (device, `tiles` entries) the tiles are tile_map[0 ..]
-// instead of [tile_base, tile_base + tiles).
-void launch_keys(const LaunchCtx &L, uint32_t *keys, uint32_t *vals, uint32_t *ids, int fresh_ids,
-                 uint32_t tiles, uint32_t tile_base, const SceneMask *fresh = nullptr,
-                 const uint32_t *tile_map = nullptr);
+// Sort keys of every tile, or of the tiles tile_map[0 .. tiles) (device), into
+// s.keys[0] from index 0, with the totals of their 8-bit digits below
+// `bits`.  Body ids (caller order) are written too for every scene
+// (fresh_ids 1) or for the scenes set in *fresh (fresh_ids 2).  `clear`:
+// tree buffers to zero meanwhile.
+struct ClearTree {
+  uint4 *buf[4];   // 16-byte words
+  uint32_t words;  // of each buffer
+};
+void launch_keys(const LaunchCtx &L, const SortScratch &s, uint32_t bits, uint32_t *ids, int fresh_ids,
+                 uint32_t tiles, const SceneMask *fresh = nullptr, const uint32_t *tile_map = nullptr,
+                 const ClearTree *clear = nullptr);
 // Permute the bodies of tiles [tile_base, tile_base + tiles) (perm from index 0),
 // or of the tiles tile_map[0 ..] (each scene's tiles among themselves).
 // With `pos_out`, also writes each permuted body's position float4 there.
@@ -207,16 +221,11 @@ uint32_t body_ctas_per_sm();
 }  // namespace fast
 
 // LSD radix sort of (key, value) pairs, 8-bit digits (kernels_sort.cu).
-struct SortScratch {
-  uint32_t *keys[2];
-  uint32_t *vals[2];
-  uint32_t *hist;     // 256 * sort tiles
-  uint32_t *totals;   // 256
-  uint32_t capacity;  // elements
-};
-uint32_t sort_tiles(uint32_t n);
-// Sorts keys[0]/vals[0] over `bits` low bits; returns which buffer holds the result.
-int radix_sort(cudaStream_t stream, SortScratch &s, uint32_t n, uint32_t bits);
+// Look-back words a sort of up to `capacity` elements may use: 256 per tile.
+size_t sort_status_words(uint32_t capacity);
+// Sorts keys[0] (written by launch_keys with the same digits and tile map) over
+// `bits` low bits; returns which buffer holds the result.  Values are slots.
+int radix_sort(const LaunchCtx &L, SortScratch &s, uint32_t n, uint32_t bits, const uint32_t *tile_map = nullptr);
 // Leaf counting sort of every scene's bodies (part_in/ids_in -> part_out/
 // ids_out) from the leaf counts in `counts` (moments of the current
 // positions).  block_scratch: leaf_sort_blocks(max_depth) words per scene;

@@ -67,6 +67,15 @@ enum DeviceError : uint32_t {
   kDevErrNone = 0,
   kDevErrTmaTimeout = 1,     // an mbarrier wait for a bulk tensor copy gave up
   kDevErrListOverflow = 2,   // a work list exceeded its capacity
+  kDevErrSortTimeout = 3,    // a sort tile's wait for its predecessors gave up
+};
+
+// State of the radix sort between passes: zero before the first one, and
+// left ready for the next by every pass.
+struct SortState {
+  uint32_t ticket;  // next tile number
+  uint32_t done;    // finished tiles
+  uint32_t epoch;   // passes so far (tags the tiles' published counts)
 };
 
 // One M2L/L2L work item: a parent cell whose count exceeds the adaptive leaf

@@ -158,3 +158,20 @@ def test_p2p_unit_edges_and_unusual_bodies_bit_exact(rfmm_mod, oracle_mod, n, so
         s.upload(p)
         s.step(1)
         _same_or_nan(s.particles(), st.particles, "particles")
+
+
+@pytest.mark.parametrize("n", [1, 1023, 1024, 1025, 65537, 311296, 311297])
+def test_sort_tile_edges_bit_exact(rfmm_mod, oracle_mod, n):
+    """The pair sums follow the stable leaf order, so they check the sort: tile
+    remainders, and both sides of the change of tile size (304 tiles of 1,024)."""
+    O, R = oracle_mod, rfmm_mod
+    from rfmm import scenes
+    p = scenes.make("uniform", n, 48)
+    st = O.OracleState(p, O.make_params(n, gravity=1.0, softening=1e-3, dt=5e-4, near_mode=1))
+    st.step(2)
+    with R.Solver(n, R.default_params(gravity=1.0, softening=1e-3, dt=5e-4)) as s:
+        s.set_near_mode(R.NEAR_P2P)
+        s.upload(p)
+        s.step(2)
+        _same(s.particles(), st.particles, "particles")
+        assert s.device_error() == (0, 0)
