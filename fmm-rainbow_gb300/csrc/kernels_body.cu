@@ -23,10 +23,9 @@ RFMM_KERNEL_NS_BEGIN
 
 // Leaf (level `depth`) cell of a position, local to the scene's tree.
 __device__ __forceinline__ uint32_t leaf_cell(float x, float y, float z, uint32_t depth) {
-  const uint32_t dim = 1u << depth;
-  return level_offset_d(depth) + lin3_lv(cell_of_unit(unit_coord(x), dim),
-                                         cell_of_unit(unit_coord(y), dim),
-                                         cell_of_unit(unit_coord(z), dim), depth);
+  uint32_t cx, cy, cz;
+  cells_of_position(x, y, z, depth, cx, cy, cz);
+  return level_offset_d(depth) + lin3_lv(cx, cy, cz, depth);
 }
 
 // 3-D Morton interleave of leaf coordinates (x in bit 0).
@@ -44,7 +43,7 @@ __device__ __forceinline__ uint32_t morton3(uint32_t x, uint32_t y, uint32_t z) 
 }
 
 __device__ __forceinline__ float length3(float x, float y, float z) {
-  return sqrtf((x * x + y * y) + z * z);
+  return sqrt_sum((x * x + y * y) + z * z);
 }
 
 // Soft absorbing band and last-resort clamp for one axis (wgsl:740-751).
@@ -84,10 +83,7 @@ __device__ __forceinline__ uint32_t sample_cell(const SceneDesc &S, float px, fl
                                                 uint32_t &lz) {
   const uint32_t D = S.depth;
   // Leaf coordinates; floor(u * 2^l) == floor(u * 2^D) >> (D - l).
-  const uint32_t dimD = 1u << D;
-  lx = cell_of_unit(unit_coord(px), dimD);
-  ly = cell_of_unit(unit_coord(py), dimD);
-  lz = cell_of_unit(unit_coord(pz), dimD);
+  cells_of_position(px, py, pz, D, lx, ly, lz);
   uint32_t chosen = D, cell_index = 0u;
   const uint32_t pick = __ldg(&choice[S.cell_off + level_offset_d(D) + lin3_lv(lx, ly, lz, D)]);
   if (pick != kChoiceUnresolved) {
@@ -393,10 +389,7 @@ __global__ void __launch_bounds__(256, 6) k_integrate(const SceneDesc *__restric
   // The next tile's bodies are loaded one iteration ahead.
   float4 n0 = make_float4(0.f, 0.f, 0.f, 0.f), n1 = n0;
   uint32_t next_tile = i < end ? (tile_list != nullptr ? tile_list[i] : i) : 0u;
-  if (i < end) {
-    n0 = part[2u * (next_tile * kTile + threadIdx.x)];
-    n1 = part[2u * (next_tile * kTile + threadIdx.x) + 1u];
-  }
+  if (i < end) load_body(part, next_tile * kTile + threadIdx.x, n0, n1);
   while (i < end) {
     const uint32_t tile = next_tile;
     const uint32_t slot = tile * kTile + threadIdx.x;
@@ -404,8 +397,7 @@ __global__ void __launch_bounds__(256, 6) k_integrate(const SceneDesc *__restric
     const uint32_t ni = dynamic ? grab() : static_tile(++k);
     if (ni < end) {
       next_tile = tile_list != nullptr ? tile_list[ni] : ni;
-      n0 = part[2u * (next_tile * kTile + threadIdx.x)];
-      n1 = part[2u * (next_tile * kTile + threadIdx.x) + 1u];
+      load_body(part, next_tile * kTile + threadIdx.x, n0, n1);
     }
     i = ni;
     // The CTA's last tile: the next step's upward pass may launch now (it
@@ -423,8 +415,7 @@ __global__ void __launch_bounds__(256, 6) k_integrate(const SceneDesc *__restric
     if (active) {
       const P2PView V{pos4, starts, slot, near4};
       integrate_body<kP2P>(S, p0, p1, mom, src, aux, choice, fields, key, qx, qy, qz, &V);
-      part[2u * slot] = p0;
-      part[2u * slot + 1u] = p1;
+      store_body(part, slot, p0, p1);
     }
     if (!kP2P) deposit_body(T, key, active, qx, qy, qz, mom_next);
   }
@@ -1113,10 +1104,10 @@ __global__ void __launch_bounds__(256) k_keys(const SceneDesc *__restrict__ scen
       // input, caller, order), else a fine cell; floor(u * 2^F) >> (F - depth)
       // == floor(u * 2^depth), so the fine key refines the leaf key.
       const float4 p = part[2u * slot];
-      const uint32_t level = S.near_mode == kNearP2P ? S.depth : F, dim = 1u << level;
-      key = S.key_base | (morton3(cell_of_unit(unit_coord(p.x), dim), cell_of_unit(unit_coord(p.y), dim),
-                                  cell_of_unit(unit_coord(p.z), dim))
-                          << (3u * (F - level)));
+      const uint32_t level = S.near_mode == kNearP2P ? S.depth : F;
+      uint32_t cx, cy, cz;
+      cells_of_position(p.x, p.y, p.z, level, cx, cy, cz);
+      key = S.key_base | (morton3(cx, cy, cz) << (3u * (F - level)));
     }
     keys[i * kTile + threadIdx.x] = key;
     for (uint32_t d = 0; d < digits; d++) atomicAdd(&s_total[d][(key >> (8u * d)) & 255u], 1u);
@@ -1168,9 +1159,9 @@ __global__ void __launch_bounds__(256) k_gather(const SceneDesc *__restrict__ sc
     // Defensive: a permutation never leaves its range (or its scene).
     if (tile_map != nullptr ? tile_scene[from / kTile] != tile_scene[tile] : (from < lo || from >= hi))
       from = slot;
-    const float4 p0 = part_in[2u * from], p1 = part_in[2u * from + 1u];
-    part_out[2u * slot] = p0;
-    part_out[2u * slot + 1u] = p1;
+    float4 p0, p1;
+    load_body(part_in, from, p0, p1);
+    store_body(part_out, slot, p0, p1);
     ids_out[slot] = ids_in[from];
     if (pos_out != nullptr) pos_out[slot] = p0;
     if (deposit_into != nullptr) {
@@ -1214,9 +1205,9 @@ __global__ void __launch_bounds__(256) k_unpermute(const SceneDesc *__restrict__
   if (slot - S.body_off >= n) return;
   const uint32_t id = ids[slot];
   if (id >= n) return;  // defensive: ids are a permutation of 0..n-1
-  const uint32_t dst = S.body_off + id;
-  out[2u * dst] = part[2u * slot];
-  out[2u * dst + 1u] = part[2u * slot + 1u];
+  float4 a, b;
+  load_body(part, slot, a, b);
+  store_body(out, S.body_off + id, a, b);
 }
 
 // ------------------------------------------------------ galaxy seeding

@@ -474,13 +474,11 @@ __global__ void __launch_bounds__(256) k_leaf_scatter(const SceneDesc *__restric
         const SceneDesc &S = scenes[tile_scene[tile]];
         const uint32_t slot = tile * 256u + threadIdx.x;
         if (slot - S.body_off < S.n) {
-          p0[r] = part_in[2u * slot];
-          p1[r] = part_in[2u * slot + 1u];
+          load_body(part_in, slot, p0[r], p1[r]);
           src[r] = slot;
-          const uint32_t dim = 1u << S.depth;
-          key = S.cell_off + (spread3s(cell_of_unit(unit_coord(p0[r].x), dim)) |
-                              (spread3s(cell_of_unit(unit_coord(p0[r].y), dim)) << 1) |
-                              (spread3s(cell_of_unit(unit_coord(p0[r].z), dim)) << 2));
+          uint32_t cx, cy, cz;
+          cells_of_position(p0[r].x, p0[r].y, p0[r].z, S.depth, cx, cy, cz);
+          key = S.cell_off + (spread3s(cx) | (spread3s(cy) << 1) | (spread3s(cz) << 2));
         }
       }
       const uint32_t peers = __match_any_sync(0xFFFFFFFFu, key);
@@ -508,8 +506,7 @@ __global__ void __launch_bounds__(256) k_leaf_scatter(const SceneDesc *__restric
       if (src[r] == kEmptyKey) continue;
       const uint32_t dst = hcnt[hs[r]] + off[r];
       if (dst >= tiles * 256u) continue;  // defensive: counts and positions always agree
-      part_out[2u * dst] = p0[r];
-      part_out[2u * dst + 1u] = p1[r];
+      store_body(part_out, dst, p0[r], p1[r]);
       ids_out[dst] = ids_in[src[r]];
     }
     if (kList) __syncthreads();  // the table is cleared for the next unit
