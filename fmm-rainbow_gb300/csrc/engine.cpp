@@ -1468,10 +1468,10 @@ int Engine::render(uint32_t scene, const rfmm_render_params &p, void *dst, size_
     out = d_render_out_;
   }
   LaunchCtx L = ctx(mcur_, lpar_, pcur_);
-  launch_slot_of(L, d_ids_[pcur_], d_slot_of_, d.tile_off, pad_tiles(d.n));
-  launch_render(L, scene, d_slot_of_, cam, d_render_acc_, d_render_tex_, d_render_tex_ + texels, out);
+  launch_render(L, scene, d.n, d_ids_[pcur_], d_slot_of_, cam, d_render_acc_, d_render_tex_, d_render_tex_ + texels,
+                out);
   RF_CK(cudaGetLastError());
-  launches_ += 5;
+  launches_ += 4;
   if (kind != cudaMemcpyDeviceToDevice)
     RF_CK(cudaMemcpyAsync(dst, out, bytes, cudaMemcpyDeviceToHost, stream_));
   return sync();

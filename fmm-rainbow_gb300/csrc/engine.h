@@ -240,7 +240,7 @@ class Engine {
   float4 *d_accphi_ = nullptr;    // diagnostics: per-body acceleration + potential
   double *d_diag_ = nullptr;      // diagnostics: FP64 partial sums
   size_t diag_doubles_ = 0;
-  uint32_t *d_slot_of_ = nullptr;  // diagnostics / render: caller id -> resident slot
+  uint32_t *d_slot_of_ = nullptr;  // by caller id: resident slot (diagnostics), draws (render)
   unsigned long long *d_render_acc_ = nullptr;  // render: fixed-point accumulation
   float4 *d_render_tex_ = nullptr;              // render: two blur textures
   uchar4 *d_render_out_ = nullptr;              // render: staging for host copies

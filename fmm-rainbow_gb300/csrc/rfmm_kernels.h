@@ -188,11 +188,9 @@ struct RenderCamera {
   float point_size;          // outer blur radius in canvas pixels
   float population_scale;    // 0.62 * (2^20 / instances)^0.14
 };
-void launch_render(const LaunchCtx &L, uint32_t scene, const uint32_t *slot_of, const RenderCamera &cam,
-                   unsigned long long *acc, float4 *tex_a, float4 *tex_b, uchar4 *out);
-// slot_of[body_off + id] = resident slot, for the bodies of tiles [tile_base, +tiles).
-void launch_slot_of(const LaunchCtx &L, const uint32_t *ids, uint32_t *slot_of, uint32_t tile_base,
-                    uint32_t tiles);
+// `ids`: caller ids of the resident slots; `counts`: n words of scratch.
+void launch_render(const LaunchCtx &L, uint32_t scene, uint32_t n, const uint32_t *ids, uint32_t *counts,
+                   const RenderCamera &cam, unsigned long long *acc, float4 *tex_a, float4 *tex_b, uchar4 *out);
 
 // FP64 diagnostics (kernels_diag.cu).
 void launch_direct_sum_f64(cudaStream_t stream, const float4 *part_caller, uint32_t n,
