@@ -101,9 +101,7 @@ int rfmm_upload_particles(rfmm_handle *h, const void *host_aos, size_t bytes) {
 
 int rfmm_upload_particles_device(rfmm_handle *h, const void *device_aos, size_t bytes) {
   if (guard(h)) return RFMM_ERR_INVALID;
-  int st = h->engine->upload(0, device_aos, bytes, cudaMemcpyDeviceToDevice);
-  if (st == RFMM_OK) st = h->engine->commit();
-  return st;
+  return h->engine->upload_commit_device(device_aos, bytes);
 }
 
 int rfmm_seed_galaxy(rfmm_handle *h) {

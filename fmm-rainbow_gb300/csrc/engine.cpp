@@ -861,15 +861,15 @@ int Engine::activate_many(const std::vector<Admission> &admissions) {
   uint32_t total = 0;
   int st = upload_map(admit_map_, slots, &total, as);
   if (st != RFMM_OK) return st;
-  // Keys of the staged bodies (numbering them in caller order), one sort,
-  // cleared trees, one gather with the leaf deposit into the current buffer.
+  // Keys of the staged bodies, one sort, cleared trees, one gather (numbering
+  // them in caller order) with the leaf deposit into the current buffer.
   LaunchCtx L = ctx(mcur_, lpar_, scr);
   L.stream = as;
-  launch_keys(L, sort_, key_bits_, d_ids_[scr], 1, total, nullptr, admit_map_.dev);
+  launch_keys(L, sort_, key_bits_, nullptr, 0, total, nullptr, admit_map_.dev);
   const int r = radix_sort(L, sort_, total * kTile, key_bits_, admit_map_.dev);
   launch_clear_scenes(L, (uint32_t)scenes_.size(), which, d_mom_[mcur_], d_mom_[mcur_ ^ 1u], d_src_, d_aux_);
-  launch_gather(L, sort_.vals[r], d_part_[scr], d_ids_[scr], d_part_[cur], d_ids_[cur], d_mom_[mcur_],
-                total, 0u, nullptr, admit_map_.dev);
+  launch_gather(L, sort_.vals[r], d_part_[scr], nullptr, 0u, nullptr, d_part_[cur], d_ids_[cur], d_mom_[mcur_], total,
+                slots_, nullptr, admit_map_.dev);
   RF_CK(cudaGetLastError());
   if (as != stream_) {  // the engine stream's next kernels see the admitted slots
     RF_CK(cudaEventRecord(admit_ev_, as));
@@ -907,23 +907,50 @@ int Engine::refresh_lists() {
   return st;
 }
 
-int Engine::commit() {
+// A device buffer the kernels can read or write in place: device or managed
+// memory of this device, 32-byte aligned.
+bool Engine::usable_in_place(const void *p) const {
+  cudaPointerAttributes a{};
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    (void)cudaGetLastError();  // a failed attribute query leaves no error behind
+    return false;
+  }
+  return ((a.type == cudaMemoryTypeDevice && a.device == device_) || a.type == cudaMemoryTypeManaged) &&
+         (reinterpret_cast<uintptr_t>(p) & 31u) == 0u;
+}
+
+int Engine::upload_commit_device(const void *src, size_t bytes) {
+  if (scenes_.size() != 1u || use_lists_ || src == nullptr || bytes != 32ull * scenes_[0].n || !usable_in_place(src)) {
+    const int st = upload(0, src, bytes, cudaMemcpyDeviceToDevice);
+    return st == RFMM_OK ? commit() : st;
+  }
+  uploaded_[0] = true;
+  return commit(static_cast<const float4 *>(src));
+}
+
+int Engine::commit(const float4 *src) {
   for (bool u : uploaded_)
     if (!u) return RFMM_ERR_STATE;
   LaunchCtx L = ctx(mcur_, lpar_, pcur_);
-  // The key pass also numbers the bodies of scenes uploaded since the last
-  // commit in caller order, and clears the moment, source and record buffers
-  // that the rebuilt tree starts from (the upward pass skips subtrees that are
-  // empty in both moment buffers).
+  // Scenes uploaded since the last commit are in caller order; when all are,
+  // a body's id is its source slot's place and the key pass writes none.
+  uint32_t fresh = 0u;
+  for (uint32_t w : fresh_.bits) fresh += (uint32_t)__builtin_popcount(w);
+  const bool all_fresh = src != nullptr || fresh == scenes_.size();
+  if (src != nullptr) L.part = const_cast<float4 *>(src);  // the key pass only reads it
+  // The key pass also numbers the bodies of such scenes where ids are read,
+  // and clears the moment, source and record buffers that the rebuilt tree
+  // starts from (the upward pass skips subtrees that are empty in both moment
+  // buffers).
   const ClearTree clear{{d_mom_[mcur_], d_mom_[mcur_ ^ 1u], reinterpret_cast<uint4 *>(d_src_),
                          reinterpret_cast<uint4 *>(d_aux_)},
                         cells_};
-  launch_keys(L, sort_, key_bits_, d_ids_[pcur_], any_fresh_ ? 2 : 0, tiles_, &fresh_, nullptr, &clear);
+  launch_keys(L, sort_, key_bits_, d_ids_[pcur_], any_fresh_ && !all_fresh ? 2 : 0, tiles_, &fresh_, nullptr, &clear);
   fresh_ = SceneMask{};
   any_fresh_ = false;
   const int r = radix_sort(L, sort_, slots_, key_bits_);
-  launch_gather(L, sort_.vals[r], d_part_[pcur_], d_ids_[pcur_], d_part_[pcur_ ^ 1u],
-                d_ids_[pcur_ ^ 1u], d_mom_[mcur_], tiles_, 0u, d_pos4_);
+  launch_gather(L, sort_.vals[r], d_part_[pcur_], src, scenes_[0].n, all_fresh ? nullptr : d_ids_[pcur_],
+                d_part_[pcur_ ^ 1u], d_ids_[pcur_ ^ 1u], d_mom_[mcur_], tiles_, slots_, d_pos4_);
   launches_ += radix_sort_kernels();
   if (near_mode_ == kNearP2P) {
     launch_leaf_starts(L, sort_.keys[r], (uint32_t)scenes_.size());
@@ -955,10 +982,10 @@ void Engine::enqueue_p2p_sort(uint32_t mpar, uint32_t lpar, uint32_t ppar, uint4
   LaunchCtx L = ctx(mpar, lpar, ppar);
   launch_unpermute(L, d_ids_[ppar], d_part_[ppar ^ 1u], 0u, tiles_);
   LaunchCtx C = ctx(mpar, lpar, ppar ^ 1u);
-  launch_keys(C, sort_, key_bits_, d_ids_[ppar ^ 1u], 1, tiles_);
+  launch_keys(C, sort_, key_bits_, nullptr, 0, tiles_);
   const int r = radix_sort(C, sort_, slots_, key_bits_);
-  launch_gather(L, sort_.vals[r], d_part_[ppar ^ 1u], d_ids_[ppar ^ 1u], d_part_[ppar],
-                d_ids_[ppar], mom_into, tiles_, 0u, d_pos4_);
+  launch_gather(L, sort_.vals[r], d_part_[ppar ^ 1u], nullptr, 0u, nullptr, d_part_[ppar], d_ids_[ppar], mom_into, tiles_,
+                slots_, d_pos4_);
   launch_leaf_starts(L, sort_.keys[r], (uint32_t)scenes_.size());
 }
 
@@ -1110,9 +1137,14 @@ int Engine::step(uint32_t steps) {
 int Engine::check_device_error() {
   RF_CK(cudaMemcpyAsync(h_ctr_, d_ctr_, sizeof(Counters), cudaMemcpyDeviceToHost, stream_));
   RF_CK(cudaStreamSynchronize(stream_));
-  if (h_ctr_->error == kDevErrTmaTimeout || h_ctr_->error == kDevErrSortTimeout) return RFMM_ERR_TIMEOUT;
-  if (h_ctr_->error != 0u) return RFMM_ERR_DEVICE;
-  return RFMM_OK;
+  return reported_error();
+}
+
+// The status the pinned copy of the error word stands for.
+int Engine::reported_error() const {
+  const uint32_t e = *static_cast<volatile uint32_t *>(&h_ctr_->error);
+  if (e == kDevErrTmaTimeout || e == kDevErrSortTimeout) return RFMM_ERR_TIMEOUT;
+  return e != 0u ? RFMM_ERR_DEVICE : RFMM_OK;
 }
 
 int Engine::sync() { return check_device_error(); }
@@ -1160,6 +1192,15 @@ int Engine::download(uint32_t scene, int which, void *dst, size_t bytes, cudaMem
   if (which == RFMM_BUF_PARTICLES) {
     if (!committed_) return RFMM_ERR_STATE;
     LaunchCtx L = ctx(mcur_, lpar_, pcur_);
+    if (kind == cudaMemcpyDeviceToDevice && usable_in_place(dst)) {
+      // Straight into the caller's buffer; the launch also reports the error
+      // word, so no copy follows.
+      launch_unpermute(L, d_ids_[pcur_], static_cast<float4 *>(dst), d.tile_off, pad_tiles(d.n), nullptr, nullptr,
+                       d.body_off, &h_ctr_->error);
+      RF_CK(cudaGetLastError());
+      RF_CK(cudaStreamSynchronize(stream_));
+      return reported_error();
+    }
     launch_unpermute(L, d_ids_[pcur_], d_part_[pcur_ ^ 1u], d.tile_off, pad_tiles(d.n));
     RF_CK(cudaGetLastError());
     from = d_part_[pcur_ ^ 1u] + 2ull * d.body_off;

@@ -70,8 +70,13 @@ class Engine {
   // per scene, one synchronisation.
   int download_all(int which, void *const *dst, cudaMemcpyKind kind);
   int seed_galaxy(uint32_t scene);
-  // Sort every scene into leaf order and deposit the leaf moments.
-  int commit();
+  // Sort every scene into leaf order and deposit the leaf moments.  With `src`,
+  // the one scene's bodies are read from that device buffer (caller order)
+  // instead of the resident one.
+  int commit(const float4 *src = nullptr);
+  // upload() from device memory and commit(); a 32-byte aligned buffer of a
+  // one-scene engine is read in place.
+  int upload_commit_device(const void *src, size_t bytes);
 
   int solve_fields();
   int step(uint32_t steps);
@@ -208,6 +213,8 @@ class Engine {
   cudaEvent_t refresh_ev_ = nullptr;
   int rebuild_lists();
   int check_device_error();
+  int reported_error() const;
+  bool usable_in_place(const void *p) const;
 
   int device_ = 0;
   int sms_ = 0;

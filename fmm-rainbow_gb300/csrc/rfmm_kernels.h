@@ -137,20 +137,24 @@ struct ClearTree {
 void launch_keys(const LaunchCtx &L, const SortScratch &s, uint32_t bits, uint32_t *ids, int fresh_ids,
                  uint32_t tiles, const SceneMask *fresh = nullptr, const uint32_t *tile_map = nullptr,
                  const ClearTree *clear = nullptr);
-// Permute the bodies of tiles [tile_base, tile_base + tiles) (perm from index 0),
-// or of the tiles tile_map[0 ..] (each scene's tiles among themselves).
-// With `pos_out`, also writes each permuted body's position float4 there.
-void launch_gather(const LaunchCtx &L, const uint32_t *perm, const float4 *part_in,
-                   const uint32_t *ids_in, float4 *part_out, uint32_t *ids_out, uint4 *deposit_into,
-                   uint32_t tiles, uint32_t tile_base, float4 *pos_out = nullptr,
-                   const uint32_t *tile_map = nullptr);
+// Permute the bodies of every tile, or of the tiles tile_map[0 .. tiles) (each
+// scene's tiles among themselves), and deposit them into `deposit_into`.
+// part_in has `slots` slots; with `src` the one scene's src_n bodies are read
+// from there in caller order (32-byte aligned).  ids_in null: every source
+// slot holds the body of that place in its scene.  With `pos_out`, also writes
+// each permuted body's position float4 there.
+void launch_gather(const LaunchCtx &L, const uint32_t *perm, const float4 *part_in, const float4 *src,
+                   uint32_t src_n, const uint32_t *ids_in, float4 *part_out, uint32_t *ids_out, uint4 *deposit_into,
+                   uint32_t tiles, uint32_t slots, float4 *pos_out = nullptr, const uint32_t *tile_map = nullptr);
 // Leaf start tables of every kNearP2P scene from the sorted keys.
 void launch_leaf_starts(const LaunchCtx &L, const uint32_t *sorted_keys, uint32_t scenes);
 // Bodies of tiles [tile_base, tile_base + tiles) (or tile_map[0 ..]) back to
-// caller order: out[body_off + id] = part[slot].
+// caller order: out[body_off + id - out_base] = part[slot] (32-byte aligned);
+// error_out (mapped host memory, two words): the error word as of this launch.
 void launch_unpermute(const LaunchCtx &L, const uint32_t *ids, float4 *out, uint32_t tile_base,
                       uint32_t tiles, const uint32_t *tile_map = nullptr,
-                      const uint32_t *tile_count = nullptr);
+                      const uint32_t *tile_count = nullptr, uint32_t out_base = 0u,
+                      uint32_t *error_out = nullptr);
 // Scene descriptors desc[i] into scenes[index[i]] on `stream` (other entries untouched).
 void launch_write_scenes(cudaStream_t stream, SceneDesc *scenes, const uint32_t *index,
                          const SceneDesc *desc, uint32_t count);

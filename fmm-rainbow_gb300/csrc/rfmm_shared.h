@@ -54,7 +54,7 @@ static_assert(sizeof(SceneDesc) == 112, "SceneDesc layout");
 struct Counters {
   uint32_t parents[2];   // length of the parent work list, per step parity
   uint32_t error;        // first error code raised by a kernel (0 = none)
-  uint32_t error_info;   // kernel-specific detail for `error`
+  uint32_t error_info;   // kernel-specific detail for `error` (right behind it)
   uint32_t tiles_active; // entries of the active body-tile list (when one is used)
   uint32_t tasks_active; // entries of the active upward-task list (when one is used)
   uint32_t scenes_active; // entries of the active scene list (when one is used)
