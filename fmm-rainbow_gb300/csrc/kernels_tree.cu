@@ -619,22 +619,45 @@ constexpr uint32_t kChunk = 64u;        // stencil slots evaluated per pass (216
 constexpr uint32_t kSlotStride = 65u;   // padded so the 80 summing threads hit distinct banks
 constexpr uint32_t kTmaBytes = kTileCells * 16u;
 
-// Stencil slot k in the reference's loop order (source parent (pz, py, px),
+constexpr uint32_t kContrib = 189u;  // stencil slots not adjacent to a given child
+
+// The stencil, worked out by the compiler (as integer code in every CTA's
+// prologue it was a fifth of the one-scene kernel's instructions, and 26,000
+// serial ones in the many-scene kernel; the gap in front of M2L at 256
+// scenes went from 4.6 to 3.0 us).
+// slot[k]: slot k in the reference's loop order (source parent (pz, py, px),
 // then child (cz, cy, cx)): bits 0-7 the slot's cell in the 6x6x6 tile, bit
 // 8 + c set when the cell is adjacent to (or is) child c of the target parent.
-__device__ __forceinline__ uint16_t m2l_slot_info(uint32_t k) {
-  const uint32_t pidx = k >> 3, ch = k & 7u;
-  const int ux = 2 * (int)(pidx % 3u) + (int)(ch & 1u);
-  const int uy = 2 * (int)((pidx / 3u) % 3u) + (int)((ch >> 1) & 1u);
-  const int uz = 2 * (int)(pidx / 9u) + (int)(ch >> 2);
-  uint32_t near = 0u;
-  for (uint32_t c = 0; c < 8u; c++) {
-    // Source child coordinate minus target coordinate = u - 2 - child.
-    const int sx = ux - 2 - (int)(c & 1u), sy = uy - 2 - (int)((c >> 1) & 1u), sz = uz - 2 - (int)(c >> 2);
-    if (sx >= -1 && sx <= 1 && sy >= -1 && sy <= 1 && sz >= -1 && sz <= 1) near |= 1u << c;
+// child[c]: the slots contributing to child c, in that order, as cell offsets
+// in the 6x6x6 block (3 bits per axis).
+struct M2LStencil {
+  uint16_t slot[kTileCells];
+  uint16_t child[8][kContrib];
+  constexpr M2LStencil() : slot(), child() {
+    for (uint32_t k = 0; k < kTileCells; k++) {
+      const uint32_t pidx = k >> 3, ch = k & 7u;
+      const int ux = 2 * (int)(pidx % 3u) + (int)(ch & 1u);
+      const int uy = 2 * (int)((pidx / 3u) % 3u) + (int)((ch >> 1) & 1u);
+      const int uz = 2 * (int)(pidx / 9u) + (int)(ch >> 2);
+      uint32_t near = 0u;
+      for (uint32_t c = 0; c < 8u; c++) {
+        // Source child coordinate minus target coordinate = u - 2 - child.
+        const int sx = ux - 2 - (int)(c & 1u), sy = uy - 2 - (int)((c >> 1) & 1u), sz = uz - 2 - (int)(c >> 2);
+        if (sx >= -1 && sx <= 1 && sy >= -1 && sy <= 1 && sz >= -1 && sz <= 1) near |= 1u << c;
+      }
+      slot[k] = (uint16_t)((uint32_t)(ux + 6 * (uy + 6 * uz)) | (near << 8));
+    }
+    for (uint32_t c = 0; c < 8u; c++) {
+      uint32_t n = 0u;
+      for (uint32_t k = 0; k < kTileCells; k++) {
+        if ((slot[k] >> (8u + c)) & 1u) continue;  // adjacent to (or is) child c
+        const uint32_t t = slot[k] & 0xFFu;
+        if (n < kContrib) child[c][n++] = (uint16_t)((t % 6u) | (((t / 6u) % 6u) << 3) | ((t / 36u) << 6));
+      }
+    }
   }
-  return (uint16_t)((uint32_t)(ux + 6 * (uy + 6 * uz)) | (near << 8));
-}
+};
+static __device__ const M2LStencil kStencil = M2LStencil();
 
 struct M2LShared {
   float4 tile[kTileCells];  // first member: 128-byte aligned by the launch
@@ -710,20 +733,9 @@ __device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, i
 // reference's loop order, each adding its terms to its own ten sums (no
 // partial sum crosses lanes).  Source cells are read through L1.  `clist`
 // holds per child the contributing slots' cell offsets in the 6x6x6 block
-// (3 bits per axis), built once per CTA.
-constexpr uint32_t kContrib = 189u;
-
-__device__ __forceinline__ void build_child_slots(uint16_t (*clist)[kContrib]) {
-  if (threadIdx.x < 8u) {
-    const uint32_t c = threadIdx.x;
-    uint32_t n = 0u;
-    for (uint32_t k = 0; k < kTileCells; k++) {
-      const uint32_t info = m2l_slot_info(k);
-      if ((info >> (8u + c)) & 1u) continue;  // adjacent to (or is) child c
-      const uint32_t t = info & 0xFFu;
-      if (n < kContrib) clist[c][n++] = (uint16_t)((t % 6u) | (((t / 6u) % 6u) << 3) | ((t / 36u) << 6));
-    }
-  }
+// (3 bits per axis).
+__device__ __forceinline__ void copy_child_slots(uint16_t (*clist)[kContrib]) {
+  for (uint32_t k = threadIdx.x; k < 8u * kContrib; k += blockDim.x) (&clist[0][0])[k] = (&kStencil.child[0][0])[k];
 }
 
 __device__ __forceinline__ void m2l_lanes_pass(const SceneDesc *__restrict__ scenes,
@@ -832,8 +844,8 @@ __global__ void __launch_bounds__(256, kWide ? 4 : 6) k_m2l(const SceneDesc *__r
     sh.stop = 0u;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  for (uint32_t k = tid; k < kTileCells; k += blockDim.x) sh.slot_info[k] = m2l_slot_info(k);
-  if (kWide) build_child_slots(s_clist);
+  for (uint32_t k = tid; k < kTileCells; k += blockDim.x) sh.slot_info[k] = kStencil.slot[k];
+  if (kWide) copy_child_slots(s_clist);
   grid_dependency_wait();  // the upward pass built the tree and the parent list
   stamp_begin(stamp);
   const uint32_t count = min(ctr->parents[list_par], plist_cap);
@@ -1099,7 +1111,11 @@ __device__ __forceinline__ void l2l_lanes_pass(const SceneDesc *__restrict__ sce
 
 struct L2LShared {
   float vals[8][10][27];
-  float centre[127];  // cell_center_lv(c, l) at [2^l - 1 + c], levels 0..6
+  // At [2^l - 1 + c]: cell_center_lv(c, l) less its parent's, levels 1..6
+  // (the one subtraction the reference makes per axis, done once per CTA
+  // instead of once per target, level and axis: 5.0 -> 4.3 us at 1,048,576
+  // Plummer bodies, 7.1 -> 6.2 at as many uniform ones).
+  float delta[127];
 };
 
 template <bool kWide>
@@ -1117,7 +1133,8 @@ __global__ void __launch_bounds__(256) k_l2l_near(const SceneDesc *__restrict__ 
   const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
   if (tid < 127u) {
     const uint32_t l = 31u - (uint32_t)__clz((int)(tid + 1u));
-    sh.centre[tid] = cell_center_lv(tid + 1u - (1u << l), l);
+    const uint32_t cell = tid + 1u - (1u << l);
+    sh.delta[tid] = l == 0u ? 0.0f : cell_center_lv(cell, l) - cell_center_lv(cell >> 1, l - 1u);
   }
   grid_dependency_wait();  // M2L results of every target are complete
   stamp_begin(stamp);
@@ -1182,10 +1199,8 @@ __global__ void __launch_bounds__(256) k_l2l_near(const SceneDesc *__restrict__ 
       if (a <= l) {
         const uint32_t sh_ = l - a;
         const uint32_t ax = tx >> sh_, ay = ty >> sh_, az = tz >> sh_;
-        const float *cen = sh.centre + (1u << a) - 1u, *pcen = sh.centre + (1u << (a - 1u)) - 1u;
-        const float dx = cen[ax] - pcen[ax >> 1];
-        const float dy = cen[ay] - pcen[ay >> 1];
-        const float dz = cen[az] - pcen[az >> 1];
+        const float *delta = sh.delta + (1u << a) - 1u;
+        const float dx = delta[ax], dy = delta[ay], dz = delta[az];
         // inherited (wgsl:603-609): a += J . delta, phi -= a . delta, J unchanged:
         //   ax + ((Jxx dx + Jxy dy) + Jxz dz), ay + ((Jxy dx + Jyy dy) + Jyz dz),
         //   az + ((Jxz dx + Jyz dy) + Jzz dz), phi - ((ax dx + ay dy) + az dz)
