@@ -248,8 +248,7 @@ int Engine::create(const std::vector<SceneSpec> &specs, Engine **out) {
   if (e == cudaSuccess && E->use_lists_) e = cudaEventCreateWithFlags(&E->refresh_ev_, cudaEventDisableTiming);
   if (e == cudaSuccess) e = configure_tree_kernels();
   if (e == cudaSuccess) e = fast::configure_tree_kernels();
-  // Both variants' integrate grids must fit: the smaller resident count.
-  if (e == cudaSuccess) E->body_limit_ = std::min(body_ctas_per_sm(), fast::body_ctas_per_sm());
+  if (e == cudaSuccess) E->body_limit_ = body_ctas_per_sm();  // (the fast variant caps its own grid)
   {
     rfmm_tuning t{};
     // Many scenes: the warp-per-subtree upward gains from more CTAs than stay

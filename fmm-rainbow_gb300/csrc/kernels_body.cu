@@ -313,9 +313,15 @@ __device__ __forceinline__ void integrate_body(const SceneDesc &S, float4 &p0, f
 
     const float world_edge = kHalf * 0.985f;
     const float edge_band = 0.12f * kHalf;
-    soft_wall(px, vx, world_edge, edge_band);
-    soft_wall(py, vy, world_edge, edge_band);
-    soft_wall(pz, vz, world_edge, edge_band);
+    // Inside the band on every axis the walls change nothing (|p| - c > 0 is
+    // |p| > c in binary32 too): one test for the three axes instead of 30
+    // instructions (22.5 -> 21.8 us at 1,048,576 Plummer bodies, 95.5 -> 92.3
+    // at 5,242,880 clustered, 336 -> 324 at 256 scenes).
+    if (fmaxf(fmaxf(fabsf(px), fabsf(py)), fabsf(pz)) > world_edge - edge_band) {
+      soft_wall(px, vx, world_edge, edge_band);
+      soft_wall(py, vy, world_edge, edge_band);
+      soft_wall(pz, vz, world_edge, edge_band);
+    }
     constexpr float kWidth = 0.70f - 0.30f, kWidthRcp = 0x1.400002p+1f;  // RN(1 / kWidth)
     const float st = clampf_d(div_by_const(exc - 0.30f, kWidth, kWidthRcp), 0.0f, 1.0f);
     const float hue_drift = 1.0f - st * st * (3.0f - 2.0f * st);
@@ -341,10 +347,18 @@ __device__ __forceinline__ void integrate_body(const SceneDesc &S, float4 &p0, f
 //
 // kP2P: near field by exact pair sums over the leaf-sorted position snapshot;
 // no deposit (the end-of-step sort deposits the new positions).
-// Six resident CTAs per SM (40 registers): more warps to cover the latency of
-// the per-body dependent chain (measured: 6 CTAs beat 4 and 8).
+// Resident CTAs per SM: six in the exact contract (40 registers; 6 / 5 at
+// 1,048,576 Plummer bodies 21.8 / 22.9 us, 5,242,880 clustered 92.3 / 94.8,
+// 256 scenes 324 / 331: more warps cover the per-body dependent chain), five
+// in the fast variant, whose shorter chains gain more from the registers
+// (20.1 / 19.2 and 76.7 / 75.0 us).
+#ifdef RFMM_FAST_FLOAT
+constexpr uint32_t kIntegrateCtas = 5u;
+#else
+constexpr uint32_t kIntegrateCtas = 6u;
+#endif
 template <bool kP2P>
-__global__ void __launch_bounds__(256, 6) k_integrate(const SceneDesc *__restrict__ scenes,
+__global__ void __launch_bounds__(256, kIntegrateCtas) k_integrate(const SceneDesc *__restrict__ scenes,
                                                    const uint32_t *__restrict__ tile_scene,
                                                    float4 *__restrict__ part,
                                                    const uint4 *__restrict__ mom,
@@ -363,8 +377,12 @@ __global__ void __launch_bounds__(256, 6) k_integrate(const SceneDesc *__restric
   __shared__ SceneDesc S;
   __shared__ uint32_t s_next;
   if (!kP2P) T.clear();
-  grid_dependency_wait();  // fields of this step are complete
-  stamp_begin(stamp);
+  // Before the wait for this step's fields: the tile lists and scene
+  // descriptors change only by host copies, and the bodies were last written
+  // by a launch that was complete before the tree passes between began their
+  // work (each of them waited for its predecessor), so the first tile's
+  // descriptor and bodies are loaded while those passes drain (a step 0.2 to
+  // 0.5 us shorter).
   const uint32_t ntiles = tile_list != nullptr ? min(ctr->tiles_active, tiles) : tiles;
   // Static schedule: interleaved tiles.  Dynamic: tiles are taken one at a
   // time from a counter (reset by this step's upward pass).
@@ -384,12 +402,19 @@ __global__ void __launch_bounds__(256, 6) k_integrate(const SceneDesc *__restric
   auto static_tile = [&](uint32_t kk) {
     return (((kk >> run_log2) * gridDim.x + blockIdx.x) << run_log2) + (kk & ((1u << run_log2) - 1u));
   };
+  if (dynamic) grid_dependency_wait();  // its counter belongs to the tree passes
   uint32_t i = dynamic ? grab() : static_tile(k);
   uint32_t cur = 0xFFFFFFFFu;
   // The next tile's bodies are loaded one iteration ahead.
   float4 n0 = make_float4(0.f, 0.f, 0.f, 0.f), n1 = n0;
   uint32_t next_tile = i < end ? (tile_list != nullptr ? tile_list[i] : i) : 0u;
-  if (i < end) load_body(part, next_tile * kTile + threadIdx.x, n0, n1);
+  if (i < end) {
+    load_body(part, next_tile * kTile + threadIdx.x, n0, n1);
+    cur = tile_scene[next_tile];
+    load_scene(S, scenes, cur);
+  }
+  grid_dependency_wait();  // fields of this step are complete
+  stamp_begin(stamp);
   while (i < end) {
     const uint32_t tile = next_tile;
     const uint32_t slot = tile * kTile + threadIdx.x;
@@ -1346,7 +1371,9 @@ static uint32_t body_grid(const LaunchCtx &L, uint32_t tiles) {
 }
 
 void launch_integrate(const LaunchCtx &L, uint32_t tiles) {
-  launch_step_kernel(L, L.p2p ? k_integrate<true> : k_integrate<false>, dim3(body_grid(L, tiles)),
+  static const uint32_t per_sm = body_ctas_per_sm();
+  const uint32_t grid = body_grid(L, tiles), wave = L.sms * per_sm;
+  launch_step_kernel(L, L.p2p ? k_integrate<true> : k_integrate<false>, dim3(grid < wave ? grid : wave),
                      dim3(kTile), 0, L.scenes, L.tile_scene, L.part, (const uint4 *)L.mom,
                      (const float4 *)L.src, (const float4 *)L.aux, (const uint32_t *)L.choice,
                      (const float *)L.fields, L.mom_next, tiles, L.tile_list, L.ctr,
