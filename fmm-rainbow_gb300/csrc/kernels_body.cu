@@ -489,8 +489,8 @@ __global__ void __launch_bounds__(256, kIntegrateCtas) k_integrate(const SceneDe
 // source: one such warp used to end the launch).
 //
 // Measured, ms per launch, one CTA per 256 slots with IEEE 1/sqrt before ->
-// now: Plummer 1,048,576 exact 167 -> 108, fast 88 -> 60; Plummer 120,001
-// exact 50 -> 8.8; clusters 600,007 fast 26 -> 15.
+// now: Plummer 1,048,576 exact 167 -> 102, fast 88 -> 55; Plummer 120,001
+// exact 50 -> 6.7; clusters 600,007 fast 26 -> 11.7.
 
 constexpr uint32_t kP2PChunk = 128u;       // sources per staged chunk: four per lane
 constexpr uint32_t kP2PWarps = 4u;         // warps per CTA (independent)
@@ -500,6 +500,13 @@ constexpr uint32_t kP2PBodies = 2u;        // bodies per lane
 #else
 constexpr uint32_t kP2PBodies = 1u;
 #endif
+// Resident CTAs per SM.  Exact, unsplit: with 16 sources in flight three warps
+// per sub-partition fill the pipe, and fewer units are half done when the
+// last are taken (3 / 4 CTAs with 16 sources, 4 with 8, ms: Plummer 120,001
+// 6.7 / 7.1 / 7.5, 1,048,576 102 / 104 / 108, clusters 600,007 21.6 / 21.8 /
+// 24.6); the fast variant needs four (3 / 4: Plummer 120,001 3.7 / 3.4).
+template <uint32_t kSplit>
+constexpr uint32_t kP2PCtas = kSplit == 1u && kP2PBodies == 1u ? 3u : 4u;
 template <uint32_t kSplit>
 constexpr uint32_t kP2PUnit = 32u / kSplit * kP2PBodies;  // slots per work unit
 // Two binary32 values in a 64-bit register pair; every operation rounds each
@@ -736,7 +743,7 @@ __device__ __forceinline__ void p2p_pass(P2PStage &T, P2PTerms &U, const float4 
     }
 #else
     if constexpr (kSplit == 1u) {
-#pragma unroll 2
+#pragma unroll 4
       for (uint32_t k = 0; k < m; k += 4u) {
         const ulonglong2 qx = *reinterpret_cast<const ulonglong2 *>(&T.x[k]);
         const ulonglong2 qy = *reinterpret_cast<const ulonglong2 *>(&T.y[k]);
@@ -816,7 +823,7 @@ __device__ __forceinline__ void p2p_pass(P2PStage &T, P2PTerms &U, const float4 
 }
 
 template <uint32_t kSplit>
-__global__ void __launch_bounds__(32 * kP2PWarps, 4) k_near_p2p(const SceneDesc *__restrict__ scenes,
+__global__ void __launch_bounds__(32 * kP2PWarps, kP2PCtas<kSplit>) k_near_p2p(const SceneDesc *__restrict__ scenes,
                                                   const uint32_t *__restrict__ tile_scene,
                                                   const float4 *__restrict__ pos4,
                                                   const uint32_t *__restrict__ starts,
@@ -848,6 +855,11 @@ __global__ void __launch_bounds__(32 * kP2PWarps, 4) k_near_p2p(const SceneDesc 
     if (lane == 0u) unit = atomicAdd(&ctr->p2p_cursor, 1u);
     unit = __shfl_sync(kAll, unit, 0);
     if (unit >= nunits) break;
+    // From both ends of the slots inwards: the ends of the Morton order hold
+    // the outlying bodies, whose warps take longest (last, they ended the
+    // launch: Plummer 120,001 exact 8.7 -> 7.5 ms, clusters 600,007 31.9 ->
+    // 24.6, fast 15.4 -> 11.7).
+    unit = (unit & 1u) ? nunits - 1u - (unit >> 1) : unit >> 1;
     const uint32_t entry = unit / kUnitsPerTile;
     const uint32_t tile = tile_list != nullptr ? tile_list[entry] : entry;
     const SceneDesc &S = scenes[tile_scene[tile]];
@@ -1401,11 +1413,11 @@ static void launch_near_p2p_split(const LaunchCtx &L, uint32_t tiles) {
 
 void launch_near_p2p(const LaunchCtx &L, uint32_t tiles) {
   // Units of 8 bodies while units of 32 would leave warps idle: up to 8 per
-  // SM (38,912 slots on 152).  Exact, ms, 8 / 32: Plummer 16,384 0.55 / 0.68,
-  // 32,768 1.79 / 1.78, 120,001 9.6 / 8.8; uniform 16,384 0.13 / 0.18.  The
-  // fast variant's split costs nothing, so it always takes 16 (16 / 64:
-  // Plummer 16,384 0.33 / 0.76, 1,048,576 59.8 / 54.6, clusters 600,007
-  // 15.0 / 24.2).
+  // SM (38,912 slots on 152).  Exact, ms, 8 / 32, in slot order: Plummer
+  // 16,384 0.55 / 0.68, 32,768 1.79 / 1.78, 120,001 9.6 / 8.8; uniform 16,384
+  // 0.13 / 0.18.  The fast variant's split costs nothing, so it always takes
+  // 16 (16 / 64, in slot order: Plummer 16,384 0.33 / 0.76, 1,048,576 59.8 /
+  // 54.6, clusters 600,007 15.0 / 24.2).
 #ifdef RFMM_FAST_FLOAT
   launch_near_p2p_split<4>(L, tiles);
 #else
