@@ -1031,11 +1031,21 @@ int Engine::solve_fields() {
 }
 
 int Engine::launch_chunk(uint32_t len, bool sort_at_end) {
-  Graph *g = nullptr;
-  const int st = capture_chunk(len, mcur_, lpar_, pcur_.load(), sort_at_end, &g);
-  if (st != RFMM_OK) return st;
-  RF_CK(cudaGraphLaunch(g->exec, stream_));
-  launches_ += g->kernels;
+  if (len == 1u && near_mode_ == kNearReference && !timeline_ && !use_lists_) {
+    // A lone step of four launches: launched directly they chain to the work
+    // before them like the steps inside a graph do, and nothing is captured
+    // for a first step (4,096 bodies, one frame: 48 us as a graph).
+    enqueue_step(mcur_, lpar_, pcur_);
+    if (sort_at_end) enqueue_resort(pcur_, mcur_ ^ 1u);
+    RF_CK(cudaGetLastError());
+    launches_ += kernels_per_step() + (sort_at_end ? resort_kernels() : 0u);
+  } else {
+    Graph *g = nullptr;
+    const int st = capture_chunk(len, mcur_, lpar_, pcur_.load(), sort_at_end, &g);
+    if (st != RFMM_OK) return st;
+    RF_CK(cudaGraphLaunch(g->exec, stream_));
+    launches_ += g->kernels;
+  }
   const uint32_t flip = len & 1u;
   tree_buf_ = (int)(mcur_ ^ ((len - 1u) & 1u));
   mcur_ ^= flip;
@@ -1209,6 +1219,12 @@ int Engine::download(uint32_t scene, int which, void *dst, size_t bytes, cudaMem
   } else {
     if (!solved_) return RFMM_ERR_STATE;
     from = d_fields_ + 12ull * d.cell_off;
+  }
+  if (kind == cudaMemcpyDeviceToDevice && usable_in_place(dst)) {
+    launch_copy_out(ctx(mcur_, lpar_, pcur_), from, dst, bytes, &h_ctr_->error);
+    RF_CK(cudaGetLastError());
+    RF_CK(cudaStreamSynchronize(stream_));
+    return reported_error();
   }
   RF_CK(cudaMemcpyAsync(dst, from, bytes, kind, stream_));
   return sync();
@@ -1497,6 +1513,7 @@ int Engine::render(uint32_t scene, const rfmm_render_params &p, void *dst, size_
     if (st == RFMM_OK) st = alloc((void **)&d_render_tex_, 32ull * texels);
     if (st != RFMM_OK) return st;
     render_texels_ = texels;
+    render_clear_ = false;
   }
   uchar4 *out = reinterpret_cast<uchar4 *>(dst);
   if (kind != cudaMemcpyDeviceToDevice) {
@@ -1508,13 +1525,19 @@ int Engine::render(uint32_t scene, const rfmm_render_params &p, void *dst, size_
     out = d_render_out_;
   }
   LaunchCtx L = ctx(mcur_, lpar_, pcur_);
+  // Every frame leaves the sums it used at zero; a fresh array, or a frame
+  // that could not be launched whole, is cleared first.
+  if (!render_clear_) RF_CK(cudaMemsetAsync(d_render_acc_, 0, 32ull * render_texels_, stream_));
+  render_clear_ = false;
   launch_render(L, scene, d.n, d_ids_[pcur_], d_slot_of_, cam, d_render_acc_, d_render_tex_, d_render_tex_ + texels,
-                out);
+                out, &h_ctr_->error);
   RF_CK(cudaGetLastError());
+  render_clear_ = true;
   launches_ += 4;
   if (kind != cudaMemcpyDeviceToDevice)
     RF_CK(cudaMemcpyAsync(dst, out, bytes, cudaMemcpyDeviceToHost, stream_));
-  return sync();
+  RF_CK(cudaStreamSynchronize(stream_));
+  return reported_error();
 }
 
 int Engine::diagnostics(uint32_t scene, double out[9]) {

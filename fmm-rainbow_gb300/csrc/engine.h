@@ -252,6 +252,7 @@ class Engine {
   float4 *d_render_tex_ = nullptr;              // render: two blur textures
   uchar4 *d_render_out_ = nullptr;              // render: staging for host copies
   size_t render_texels_ = 0, render_pixels_ = 0;
+  bool render_clear_ = false;  // every sum of d_render_acc_ is zero
   int diag_prepare(uint32_t scene, size_t doubles, bool all_bodies);
   float4 *d_src_ = nullptr;
   float4 *d_aux_ = nullptr;

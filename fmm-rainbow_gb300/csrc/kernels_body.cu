@@ -1225,6 +1225,20 @@ __global__ void __launch_bounds__(256) k_gather(const SceneDesc *__restrict__ sc
   T.flush(deposit_into);
 }
 
+// Copy of a result buffer with the error word behind it (k_unpermute's
+// error_out): one launch where a copy and a second copy of the word ran.
+__global__ void __launch_bounds__(256) k_copy_out(const uint4 *__restrict__ from, uint4 *__restrict__ to, uint32_t words,
+                                                  const Counters *__restrict__ ctr, volatile uint32_t *error_out) {
+  report_error(ctr, error_out);
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < words; i += gridDim.x * blockDim.x) to[i] = from[i];
+}
+
+void launch_copy_out(const LaunchCtx &L, const void *from, void *to, size_t bytes, uint32_t *error_out) {
+  const uint32_t words = (uint32_t)(bytes / 16u), ctas = (words + 255u) / 256u;
+  k_copy_out<<<ctas < 16u * L.sms ? ctas : 16u * L.sms, 256, 0, L.stream>>>(static_cast<const uint4 *>(from),
+                                                                          static_cast<uint4 *>(to), words, L.ctr, error_out);
+}
+
 // Scatter bodies back to the caller's order: out[body_off + id - out_base] =
 // part[slot].  With `error_out` (mapped host memory) the engine's error word
 // and its detail go there too, for a caller that waits for this launch.
@@ -1237,10 +1251,7 @@ __global__ void __launch_bounds__(256) k_unpermute(const SceneDesc *__restrict__
                                                    const uint32_t *__restrict__ tile_count, uint32_t out_base,
                                                    const Counters *__restrict__ ctr,
                                                    volatile uint32_t *error_out) {
-  if (error_out != nullptr && blockIdx.x == 0u && threadIdx.x == 0u) {
-    error_out[0] = ctr->error;
-    error_out[1] = ctr->error_info;
-  }
+  report_error(ctr, error_out);
   const uint32_t tile = tile_map != nullptr ? tile_map[blockIdx.x] : tile_base + blockIdx.x;
   const SceneDesc &S = scenes[tile_scene[tile]];
   // The scene's body count: from the caller when given (a retiring serving

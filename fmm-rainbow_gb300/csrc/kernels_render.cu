@@ -255,10 +255,18 @@ __global__ void __launch_bounds__(256) k_blur(const unsigned long long *__restri
 // resolve_fragment (wgsl:972-1009) for every canvas pixel: bilinear sample of
 // the blurred field, density-normalised colour, filmic curve, gamma 0.82,
 // written as RGBA8 (row 0 = top of the canvas).
+// The pass also clears the accumulation for the next frame (its readers are
+// complete), under the arithmetic that bounds it.
 __global__ void __launch_bounds__(256) k_resolve(const float4 *__restrict__ tex, RenderCamera cam,
-                                                 uchar4 *__restrict__ out) {
+                                                 unsigned long long *__restrict__ acc, uchar4 *__restrict__ out,
+                                                 const Counters *__restrict__ ctr, volatile uint32_t *error_out) {
   const uint32_t x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
   grid_dependency_wait();
+  report_error(ctr, error_out);
+  {
+    const uint32_t sums = 4u * cam.acc_w * cam.acc_h, row = gridDim.x * blockDim.x;
+    for (uint32_t i = y * row + x; i < sums; i += gridDim.y * row) acc[i] = 0ull;
+  }
   const uint32_t W = (uint32_t)cam.canvas_w, H = (uint32_t)cam.canvas_h;
   if (x >= W || y >= H) return;
   const uint32_t w = cam.acc_w, h = cam.acc_h;
@@ -288,8 +296,8 @@ __global__ void __launch_bounds__(256) k_resolve(const float4 *__restrict__ tex,
 }
 
 void launch_render(const LaunchCtx &L, uint32_t scene, uint32_t n, const uint32_t *ids, uint32_t *counts,
-                   const RenderCamera &cam, unsigned long long *acc, float4 *tex_a, float4 *tex_b, uchar4 *out) {
-  cudaMemsetAsync(acc, 0, 32ull * cam.acc_w * cam.acc_h, L.stream);
+                   const RenderCamera &cam, unsigned long long *acc, float4 *tex_a, float4 *tex_b, uchar4 *out,
+                   uint32_t *error_out) {
   // i -> (a i + c) mod 2^32 mod n with odd a permutes 0..n-1 when n divides
   // 2^32: every body is drawn instances / n times.
   const bool even = (n & (n - 1u)) == 0u && cam.instances % n == 0u;
@@ -308,7 +316,8 @@ void launch_render(const LaunchCtx &L, uint32_t scene, uint32_t n, const uint32_
   launch_step_kernel(L, k_blur<false>, grid_a, dim3(256), 0, (const unsigned long long *)nullptr, (const float4 *)tex_a, cam,
                      1, 0u, tex_b);
   const dim3 grid_c(((uint32_t)cam.canvas_w + 255u) / 256u, (uint32_t)cam.canvas_h);
-  launch_step_kernel(L, k_resolve, grid_c, dim3(256), 0, (const float4 *)tex_b, cam, out);
+  launch_step_kernel(L, k_resolve, grid_c, dim3(256), 0, (const float4 *)tex_b, cam, acc, out, (const Counters *)L.ctr,
+                     (volatile uint32_t *)error_out);
 }
 
 }  // namespace rfmm

@@ -155,6 +155,9 @@ void launch_unpermute(const LaunchCtx &L, const uint32_t *ids, float4 *out, uint
                       uint32_t tiles, const uint32_t *tile_map = nullptr,
                       const uint32_t *tile_count = nullptr, uint32_t out_base = 0u,
                       uint32_t *error_out = nullptr);
+// `bytes` (a multiple of 16) from `from` to `to`, and the error word as of this
+// launch to error_out (mapped host memory, two words).
+void launch_copy_out(const LaunchCtx &L, const void *from, void *to, size_t bytes, uint32_t *error_out);
 // Scene descriptors desc[i] into scenes[index[i]] on `stream` (other entries untouched).
 void launch_write_scenes(cudaStream_t stream, SceneDesc *scenes, const uint32_t *index,
                          const SceneDesc *desc, uint32_t count);
@@ -192,9 +195,12 @@ struct RenderCamera {
   float point_size;          // outer blur radius in canvas pixels
   float population_scale;    // 0.62 * (2^20 / instances)^0.14
 };
-// `ids`: caller ids of the resident slots; `counts`: n words of scratch.
+// `ids`: caller ids of the resident slots; `counts`: n words of scratch;
+// `acc` must be zero and is left zero; error_out as in launch_copy_out (null:
+// not written).
 void launch_render(const LaunchCtx &L, uint32_t scene, uint32_t n, const uint32_t *ids, uint32_t *counts,
-                   const RenderCamera &cam, unsigned long long *acc, float4 *tex_a, float4 *tex_b, uchar4 *out);
+                   const RenderCamera &cam, unsigned long long *acc, float4 *tex_a, float4 *tex_b, uchar4 *out,
+                   uint32_t *error_out);
 
 // FP64 diagnostics (kernels_diag.cu).
 void launch_direct_sum_f64(cudaStream_t stream, const float4 *part_caller, uint32_t n,
