@@ -266,7 +266,7 @@ int radix_sort(const LaunchCtx &L, SortScratch &s, uint32_t n, uint32_t bits, co
 //   k_leaf_offsets     per block, exclusive scan of its counts -> first slot of
 //                      every leaf (starts, at the scene's cell offset)
 //   k_leaf_scatter     every body takes the next slot of its leaf (one atomic
-//                      per leaf group of a warp) and moves there with its id
+//                      per leaf run of a warp) and moves there with its id
 // Bodies of one leaf land in an arbitrary order, which no result depends on:
 // each body's update reads only its own state and the tree, and the moment
 // sums are exact integers.
@@ -331,7 +331,8 @@ __global__ void __launch_bounds__(kLeafThreads) k_leaf_block_sums(const SceneDes
                                                                   uint32_t max_blocks,
                                                                   unsigned long long *__restrict__ stamp) {
   __shared__ uint32_t warp_buf[32];
-  stamp_begin(stamp);  // first of the resort's four kernels
+  grid_dependency_wait();  // the deposit of the current positions is complete
+  stamp_begin(stamp);      // first of the resort's four kernels
   const uint32_t rows = scene_rows(scene_list, ctr, nscenes);
   for (uint32_t y = blockIdx.y; y < rows; y += gridDim.y) {
     const uint32_t sc = scene_list != nullptr ? scene_list[y] : y;
@@ -357,6 +358,7 @@ __global__ void __launch_bounds__(32) k_leaf_block_scan(const SceneDesc *__restr
                                                         const Counters *__restrict__ ctr,
                                                         uint32_t *__restrict__ block_sums,
                                                         uint32_t max_blocks) {
+  grid_dependency_wait();
   const uint32_t rows = scene_rows(scene_list, ctr, nscenes);
   for (uint32_t y = blockIdx.x; y < rows; y += gridDim.x) {
     const uint32_t sc = scene_list != nullptr ? scene_list[y] : y;
@@ -388,6 +390,7 @@ __global__ void __launch_bounds__(kLeafThreads) k_leaf_offsets(const SceneDesc *
                                                                uint32_t max_blocks,
                                                                uint32_t *__restrict__ starts) {
   __shared__ uint32_t warp_sums[32];
+  grid_dependency_wait();
   const uint32_t rows = scene_rows(scene_list, ctr, nscenes);
   for (uint32_t y = blockIdx.y; y < rows; y += gridDim.y) {
     const uint32_t sc = scene_list != nullptr ? scene_list[y] : y;
@@ -431,14 +434,19 @@ __global__ void __launch_bounds__(kLeafThreads) k_leaf_offsets(const SceneDesc *
   }
 }
 
-// Each CTA moves the bodies of kScatterTiles tiles at a time (every tile
-// once, or the active tiles of a tile list in turn).  Slots are reserved in
-// two levels so a dense leaf (tens of thousands of bodies) sees one global
-// atomic per CTA instead of one per warp: warp groups of a leaf reserve their
-// offsets in a shared-memory table of the CTA's leaves, then one thread per
-// leaf reserves the CTA's whole block of that leaf from `starts`.
-constexpr uint32_t kScatterTiles = 2u;
-constexpr uint32_t kScatterSlots = 2048u;  // > bodies per CTA, so probing always ends
+// Each CTA moves the bodies of one tile at a time (every tile once, or the
+// active tiles of a tile list in turn).  Slots are reserved in two levels so
+// a dense leaf (tens of thousands of bodies) sees one global atomic per CTA:
+// runs of neighbouring lanes in one leaf reserve their offsets in a
+// shared-memory table of the CTA's leaves, then one thread per leaf reserves
+// the CTA's whole block of that leaf from `starts`.  (One global atomic per
+// run instead: uniform 1,048,576 bodies 19 us per re-sort, but Plummer 152,
+// queued on the core leaves.  Two or four tiles per CTA: Plummer 23.2 and
+// 24.5, clusters 5,242,880 81 and 92.)  With the re-sort's launches chained,
+// a list of the table's used slots instead of scans over it, and lane runs
+// instead of a match, before -> now, us: Plummer 1,048,576 32.5 -> 23.2,
+// clusters 5,242,880 105 -> 80, 256 scenes 392 -> 318, uniform 65,536 14 -> 10.
+constexpr uint32_t kScatterSlots = 2u * kTile;  // > bodies per CTA, so probing always ends
 
 template <bool kList>
 __global__ void __launch_bounds__(256) k_leaf_scatter(const SceneDesc *__restrict__ scenes,
@@ -451,65 +459,74 @@ __global__ void __launch_bounds__(256) k_leaf_scatter(const SceneDesc *__restric
                                                       uint32_t *__restrict__ ids_out,
                                                       uint32_t *__restrict__ starts, uint32_t tiles,
                                                       unsigned long long *__restrict__ stamp) {
+  constexpr uint32_t kAll = 0xFFFFFFFFu, kNone = 0xFFFFFFFFu;
   __shared__ uint32_t hkey[kScatterSlots], hcnt[kScatterSlots];
-  constexpr uint32_t kEmptyKey = 0xFFFFFFFFu;
+  __shared__ uint16_t used[kTile];  // table slots in use
+  __shared__ uint32_t nused;
   const uint32_t lane = threadIdx.x & 31u;
+  for (uint32_t i = threadIdx.x; i < kScatterSlots; i += blockDim.x) {
+    hkey[i] = kNone;
+    hcnt[i] = 0u;
+  }
+  if (threadIdx.x == 0u) nused = 0u;
+  grid_dependency_wait();  // the leaves' first slots are known
   const uint32_t ntiles = kList ? min(ctr->tiles_active, tiles) : tiles;
-  // Without a list the grid has one unit per CTA: the loop runs once.
-  for (uint32_t unit = blockIdx.x; unit * kScatterTiles < ntiles; unit += kList ? gridDim.x : ntiles) {
-    for (uint32_t i = threadIdx.x; i < kScatterSlots; i += blockDim.x) {
-      hkey[i] = kEmptyKey;
-      hcnt[i] = 0u;
+  // Without a list the grid has one tile per CTA: the loop runs once.
+  for (uint32_t i = blockIdx.x; i < ntiles; i += kList ? gridDim.x : ntiles) {
+    const uint32_t tile = kList ? tile_list[i] : i;
+    const SceneDesc &S = scenes[tile_scene[tile]];
+    const uint32_t slot = tile * kTile + threadIdx.x;
+    float4 p0, p1;
+    uint32_t key = kNone, id = 0u;
+    if (slot - S.body_off < S.n) {
+      load_body(part_in, slot, p0, p1);
+      id = ids_in[slot];
+      uint32_t cx, cy, cz;
+      cells_of_position(p0.x, p0.y, p0.z, S.depth, cx, cy, cz);
+      key = S.cell_off + (spread3s(cx) | (spread3s(cy) << 1) | (spread3s(cz) << 2));
     }
-    __syncthreads();
-    float4 p0[kScatterTiles], p1[kScatterTiles];
-    uint32_t off[kScatterTiles], hs[kScatterTiles], src[kScatterTiles];
-#pragma unroll
-    for (uint32_t r = 0; r < kScatterTiles; r++) {
-      const uint32_t li = unit * kScatterTiles + r;
-      uint32_t key = kEmptyKey;
-      src[r] = kEmptyKey;
-      if (li < ntiles) {
-        const uint32_t tile = kList ? tile_list[li] : li;
-        const SceneDesc &S = scenes[tile_scene[tile]];
-        const uint32_t slot = tile * 256u + threadIdx.x;
-        if (slot - S.body_off < S.n) {
-          load_body(part_in, slot, p0[r], p1[r]);
-          src[r] = slot;
-          uint32_t cx, cy, cz;
-          cells_of_position(p0[r].x, p0[r].y, p0[r].z, S.depth, cx, cy, cz);
-          key = S.cell_off + (spread3s(cx) | (spread3s(cy) << 1) | (spread3s(cz) << 2));
-        }
+    __syncthreads();  // the table is clear
+    const uint32_t prev = __shfl_up_sync(kAll, key, 1);
+    const uint32_t heads = __ballot_sync(kAll, lane == 0u || key != prev);
+    const uint32_t head = 31u - (uint32_t)__clz((int)(heads & (kAll >> (31u - lane))));  // of this lane's run
+    uint32_t h = 0u, base = 0u;
+    if (key != kNone && lane == head) {
+      const uint32_t after = lane == 31u ? 0u : heads & (kAll << (lane + 1u));
+      h = (key * 2654435761u) >> 23;  // 9-bit multiplicative hash
+      for (uint32_t probe = 0; probe < kScatterSlots; probe++) {
+        const uint32_t was = atomicCAS(&hkey[h], kNone, key);
+        if (was == kNone) used[atomicAdd(&nused, 1u)] = (uint16_t)h;
+        if (was == kNone || was == key) break;
+        h = (h + 1u) & (kScatterSlots - 1u);
       }
-      const uint32_t peers = __match_any_sync(0xFFFFFFFFu, key);
-      const uint32_t leader = __ffs(peers) - 1u;
-      uint32_t h = 0u, base = 0u;
-      if (key != kEmptyKey && lane == leader) {
-        h = (key * 2654435761u) >> 21;  // 11-bit multiplicative hash
-        for (uint32_t probe = 0; probe < kScatterSlots; probe++) {
-          const uint32_t prev = atomicCAS(&hkey[h], kEmptyKey, key);
-          if (prev == kEmptyKey || prev == key) break;
-          h = (h + 1u) & (kScatterSlots - 1u);
-        }
-        base = atomicAdd(&hcnt[h], __popc(peers));
-      }
-      hs[r] = __shfl_sync(0xFFFFFFFFu, h, leader);
-      off[r] = __shfl_sync(0xFFFFFFFFu, base, leader) + __popc(peers & ((1u << lane) - 1u));
+      base = atomicAdd(&hcnt[h], (after != 0u ? (uint32_t)__ffs((int)after) - 1u : 32u) - lane);
     }
+    h = __shfl_sync(kAll, h, head);
+    const uint32_t off = __shfl_sync(kAll, base, head) + (lane - head);
     __syncthreads();
     // One global reservation per (CTA, leaf); hcnt becomes the CTA's first slot.
-    for (uint32_t i = threadIdx.x; i < kScatterSlots; i += blockDim.x)
-      if (hkey[i] != kEmptyKey) hcnt[i] = atomicAdd(&starts[hkey[i]], hcnt[i]);
-    __syncthreads();
-#pragma unroll
-    for (uint32_t r = 0; r < kScatterTiles; r++) {
-      if (src[r] == kEmptyKey) continue;
-      const uint32_t dst = hcnt[hs[r]] + off[r];
-      if (dst >= tiles * 256u) continue;  // defensive: counts and positions always agree
-      store_body(part_out, dst, p0[r], p1[r]);
-      ids_out[dst] = ids_in[src[r]];
+    const uint32_t leaves = nused;
+    if (threadIdx.x < leaves) {
+      const uint32_t u = used[threadIdx.x];
+      hcnt[u] = atomicAdd(&starts[hkey[u]], hcnt[u]);
     }
-    if (kList) __syncthreads();  // the table is cleared for the next unit
+    __syncthreads();
+    if (key != kNone) {
+      const uint32_t dst = hcnt[h] + off;
+      if (dst < tiles * kTile) {  // defensive: counts and positions always agree
+        store_body(part_out, dst, p0, p1);
+        ids_out[dst] = id;
+      }
+    }
+    if (kList) {  // the table is cleared for the next tile
+      __syncthreads();
+      if (threadIdx.x < leaves) {
+        const uint32_t u = used[threadIdx.x];
+        hkey[u] = kNone;
+        hcnt[u] = 0u;
+      }
+      if (threadIdx.x == 0u) nused = 0u;
+    }
   }
   stamp_end(stamp);  // last of the resort's four kernels
 }
@@ -526,22 +543,17 @@ void leaf_counting_sort(const LaunchCtx &L, uint32_t scenes, uint32_t max_depth,
   // With lists (serving slots), a few rows of CTAs walk the active scenes and
   // a persistent grid the active tiles.
   const uint32_t rows = L.scene_list != nullptr ? (scenes < 32u ? scenes : 32u) : scenes;
-  const uint32_t units = (tiles + kScatterTiles - 1u) / kScatterTiles;
-  const uint32_t scatter = L.tile_list != nullptr ? (units < 8u * L.sms ? units : 8u * L.sms) : units;
-  k_leaf_block_sums<<<dim3(nb, rows), kLeafThreads, 0, L.stream>>>(L.scenes, scenes, L.scene_list, L.ctr,
-                                                                    counts, block_scratch, nb,
-                                                                    stamp_rec(L, 4u));
-  k_leaf_block_scan<<<rows, 32, 0, L.stream>>>(L.scenes, scenes, L.scene_list, L.ctr, block_scratch, nb);
-  k_leaf_offsets<<<dim3(nb, rows), kLeafThreads, 0, L.stream>>>(L.scenes, scenes, L.scene_list, L.ctr,
-                                                                 counts, block_scratch, nb, starts);
-  if (L.tile_list != nullptr)
-    k_leaf_scatter<true><<<scatter, 256, 0, L.stream>>>(L.scenes, L.tile_scene, L.tile_list, L.ctr, part_in,
-                                                        ids_in, part_out, ids_out, starts, tiles,
-                                                        stamp_rec(L, 4u));
-  else
-    k_leaf_scatter<false><<<scatter, 256, 0, L.stream>>>(L.scenes, L.tile_scene, nullptr, L.ctr, part_in,
-                                                         ids_in, part_out, ids_out, starts, tiles,
-                                                         stamp_rec(L, 4u));
+  launch_step_kernel(L, k_leaf_block_sums, dim3(nb, rows), dim3(kLeafThreads), 0, L.scenes, scenes, L.scene_list,
+                     (const Counters *)L.ctr, counts, block_scratch, nb, stamp_rec(L, 4u));
+  launch_step_kernel(L, k_leaf_block_scan, dim3(rows), dim3(32), 0, L.scenes, scenes, L.scene_list,
+                     (const Counters *)L.ctr, block_scratch, nb);
+  launch_step_kernel(L, k_leaf_offsets, dim3(nb, rows), dim3(kLeafThreads), 0, L.scenes, scenes, L.scene_list,
+                     (const Counters *)L.ctr, counts, (const uint32_t *)block_scratch, nb, starts);
+  const uint32_t wave = 8u * L.sms;
+  launch_step_kernel(L, L.tile_list != nullptr ? k_leaf_scatter<true> : k_leaf_scatter<false>,
+                     dim3(L.tile_list != nullptr && tiles > wave ? wave : tiles), dim3(256), 0, L.scenes, L.tile_scene,
+                     L.tile_list, (const Counters *)L.ctr, part_in, ids_in, part_out, ids_out, starts, tiles,
+                     stamp_rec(L, 4u));
 }
 
 }  // namespace rfmm
