@@ -509,33 +509,6 @@ template <uint32_t kSplit>
 constexpr uint32_t kP2PCtas = kSplit == 1u && kP2PBodies == 1u ? 3u : 4u;
 template <uint32_t kSplit>
 constexpr uint32_t kP2PUnit = 32u / kSplit * kP2PBodies;  // slots per work unit
-// Two binary32 values in a 64-bit register pair; every operation rounds each
-// half to nearest.
-using f32x2 = unsigned long long;
-__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
-  f32x2 v;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
-  return v;
-}
-__device__ __forceinline__ void unpack2(f32x2 v, float &lo, float &hi) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
-  f32x2 d;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
-  f32x2 d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
-// RN(a b) as a b + (-0), signed zeros included; `mz` holds two -0 the
-// compiler cannot see through.  (mul.rn.f32x2, or -0 as a constant, feeding an
-// add.rn.f32x2 comes out contracted even under -fmad=false: measured, one r^2
-// in five rounded differently from the scalar expression.)
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b, f32x2 mz) { return fma2(a, b, mz); }
-
 // One warp's staged sources: x, y and z rows of a chunk, and the neighbour
 // ranges as a sequence (first sequence index of each range, and what to add to
 // a sequence index to get its slot).
@@ -596,25 +569,14 @@ __device__ __forceinline__ void p2p_two(f32x2 qx, f32x2 qy, f32x2 qz, const P2PB
   sz = fma2(dz, w, sz);
 }
 #else
-// The terms of two consecutive sources; inv_sqrt_in_range in packed form
-// (signs folded into the factors built from y's bit pattern).
+// The terms of two consecutive sources.
 __device__ __forceinline__ void p2p_two(f32x2 qx, f32x2 qy, f32x2 qz, const P2PBody &b, f32x2 eps2, f32x2 mz,
                                         f32x2 &tx, f32x2 &ty, f32x2 &tz) {
   const f32x2 dx = add2(qx, b.nx), dy = add2(qy, b.ny), dz = add2(qz, b.nz);
   const f32x2 r2 = add2(add2(add2(mul2(dx, dx, mz), mul2(dy, dy, mz)), mul2(dz, dz, mz)), eps2);
-  float x0, x1, g0, g1;
+  float x0, x1;
   unpack2(r2, x0, x1);
-  const float y0 = rsqrt_estimate(x0), y1 = rsqrt_estimate(x1);
-  const uint32_t u0 = __float_as_uint(y0), u1 = __float_as_uint(y1);
-  const f32x2 y = pack2(y0, y1);
-  const f32x2 nh = pack2(__uint_as_float(u0 + 0x7F800000u), __uint_as_float(u1 + 0x7F800000u));  // -y/2
-  const f32x2 up = pack2(__uint_as_float(u0 + 1u), __uint_as_float(u1 + 1u));                    // y + ulp
-  const f32x2 ny = pack2(__uint_as_float(u0 ^ 0x80000000u), __uint_as_float(u1 ^ 0x80000000u));  // -y
-  const f32x2 g = mul2(r2, y, mz);
-  unpack2(g, g0, g1);
-  const f32x2 root = fma2(pack2(__fmaf_rn(g0, g0, -x0), __fmaf_rn(g1, g1, -x1)), nh, g);
-  const f32x2 ne = fma2(root, y, pack2(-1.0f, -1.0f));  // -e
-  const f32x2 inv = fma2(ne, fma2(ne, up, ny), y);
+  const f32x2 inv = inv_sqrt2_in_range(r2, x0, x1, mz);
   const f32x2 w = mul2(mul2(inv, inv, mz), inv, mz);
   tx = mul2(dx, w, mz);
   ty = mul2(dy, w, mz);

@@ -619,8 +619,6 @@ constexpr uint32_t kChunk = 64u;        // stencil slots evaluated per pass (216
 constexpr uint32_t kSlotStride = 65u;   // padded so the 80 summing threads hit distinct banks
 constexpr uint32_t kTmaBytes = kTileCells * 16u;
 
-constexpr uint32_t kContrib = 189u;  // stencil slots not adjacent to a given child
-
 // The stencil, worked out by the compiler (as integer code in every CTA's
 // prologue it was a fifth of the one-scene kernel's instructions, and 26,000
 // serial ones in the many-scene kernel; the gap in front of M2L at 256
@@ -628,12 +626,9 @@ constexpr uint32_t kContrib = 189u;  // stencil slots not adjacent to a given ch
 // slot[k]: slot k in the reference's loop order (source parent (pz, py, px),
 // then child (cz, cy, cx)): bits 0-7 the slot's cell in the 6x6x6 tile, bit
 // 8 + c set when the cell is adjacent to (or is) child c of the target parent.
-// child[c]: the slots contributing to child c, in that order, as cell offsets
-// in the 6x6x6 block (3 bits per axis).
 struct M2LStencil {
   uint16_t slot[kTileCells];
-  uint16_t child[8][kContrib];
-  constexpr M2LStencil() : slot(), child() {
+  constexpr M2LStencil() : slot() {
     for (uint32_t k = 0; k < kTileCells; k++) {
       const uint32_t pidx = k >> 3, ch = k & 7u;
       const int ux = 2 * (int)(pidx % 3u) + (int)(ch & 1u);
@@ -646,14 +641,6 @@ struct M2LStencil {
         if (sx >= -1 && sx <= 1 && sy >= -1 && sy <= 1 && sz >= -1 && sz <= 1) near |= 1u << c;
       }
       slot[k] = (uint16_t)((uint32_t)(ux + 6 * (uy + 6 * uz)) | (near << 8));
-    }
-    for (uint32_t c = 0; c < 8u; c++) {
-      uint32_t n = 0u;
-      for (uint32_t k = 0; k < kTileCells; k++) {
-        if ((slot[k] >> (8u + c)) & 1u) continue;  // adjacent to (or is) child c
-        const uint32_t t = slot[k] & 0xFFu;
-        if (n < kContrib) child[c][n++] = (uint16_t)((t % 6u) | (((t / 6u) % 6u) << 3) | ((t / 36u) << 6));
-      }
     }
   }
 };
@@ -726,37 +713,37 @@ __device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, i
       : "memory");
 }
 
-// M2L with one lane per target (long parent lists): a CTA's 8 warps take 32
-// listed parents at a time, warp c handling child c of each (lane j: parent
-// 32g + j).  The lanes of a warp walk the same 189 contributing stencil slots
-// of child c (the 216 tile cells less the 27 adjacent to it), in the
-// reference's loop order, each adding its terms to its own ten sums (no
-// partial sum crosses lanes).  Source cells are read through L1.  `clist`
-// holds per child the contributing slots' cell offsets in the 6x6x6 block
-// (3 bits per axis).
-__device__ __forceinline__ void copy_child_slots(uint16_t (*clist)[kContrib]) {
-  for (uint32_t k = threadIdx.x; k < 8u * kContrib; k += blockDim.x) (&clist[0][0])[k] = (&kStencil.child[0][0])[k];
-}
-
+// M2L with one lane per target (long parent lists): a warp takes four listed
+// parents at a time, lane 8j + c child c of parent j.  All lanes walk the
+// 6x6x6 source cells in the reference's loop order (27 neighbour parents, then
+// their children), two cells (a row of a neighbour's children) at a time, each
+// adding its terms to its own ten sums (no partial sum crosses lanes).  A cell
+// adjacent to a lane's target counts as empty there: with G m = 0 its terms
+// are +-0, which changes no sum (sums start at +0 and never become -0).
+// The eight lanes of a parent read the same cells, so a load touches four
+// addresses.  (A warp per child number, lanes on 32 parents, needs only the
+// 189 contributing cells of that child, but each load touches up to 32 lines
+// and L1 bounds the pass: 112 us, 110 with packed terms, at 256 scenes of 4k
+// to 262k bodies against 100 us here; the fast variant 101 against 79.)
 __device__ __forceinline__ void m2l_lanes_pass(const SceneDesc *__restrict__ scenes,
                                                const WorkItem *__restrict__ plist, uint32_t count,
                                                const uint4 *__restrict__ mom,
                                                const float4 *__restrict__ src,
-                                               float *__restrict__ lfield,
-                                               const uint16_t (*clist)[kContrib]) {
-  const uint32_t lane = threadIdx.x & 31u, c = threadIdx.x >> 5;  // 256 threads: c = 0..7
-  const uint16_t *cl = clist[c];
-  const uint32_t groups = (count + 31u) / 32u;
-  for (uint32_t g = blockIdx.x; g < groups; g += gridDim.x) {
-    const uint32_t item = 32u * g + lane;
+                                               float *__restrict__ lfield, f32x2 mz) {
+  const uint32_t lane = threadIdx.x & 31u, c = lane & 7u;
+  const uint32_t wpb = blockDim.x >> 5, groups = (count + 3u) / 4u;
+  // Bit u of near[axis]: tile coordinate u (0..5) lies within one cell of the
+  // target's, 2 + its child bit.
+  const uint32_t near_x = 7u << (1u + (c & 1u)), near_y = 7u << (1u + ((c >> 1) & 1u)), near_z = 7u << (1u + (c >> 2));
+  for (uint32_t g = blockIdx.x + gridDim.x * (threadIdx.x >> 5); g < groups; g += gridDim.x * wpb) {
+    const uint32_t item = 4u * g + (lane >> 3);
     const bool valid = item < count;
     const WorkItem w = valid ? plist[item] : WorkItem{0u, 0u};
     const SceneDesc &S = scenes[w.scene];
     const uint32_t lp = w.cell == 0u ? 0u : level_of_d(w.cell);
-    const uint32_t l = lp + 1u, dim = 2u << lp;
+    const uint32_t l = lp + 1u, pdim = 1u << lp, dim = 2u << lp;
     uint32_t upx, upy, upz;
     cell_coords_lv(w.cell - level_offset_d(lp), lp, upx, upy, upz);
-    const int bx = 2 * (int)upx - 2, by = 2 * (int)upy - 2, bz = 2 * (int)upz - 2;
     const uint32_t lvl_base = S.cell_off + level_offset_d(l);
     const uint32_t tx = 2u * upx + (c & 1u), ty = 2u * upy + ((c >> 1) & 1u), tz = 2u * upz + (c >> 2);
     const uint32_t target = lvl_base + lin3(tx, ty, tz, dim);
@@ -767,47 +754,54 @@ __device__ __forceinline__ void m2l_lanes_pass(const SceneDesc *__restrict__ sce
 #pragma unroll
     for (int k = 0; k < 10; k++) acc[k] = 0.0f;
     if (__any_sync(0xFFFFFFFFu, live)) {
-      // Two consecutive slots per iteration: their pair terms are
-      // independent chains (the square root and division of one overlap the
-      // other's), and they are added in slot order.  The next two slots'
-      // sources are requested meanwhile.
-      auto fetch = [&](uint32_t k, float4 &sv) {
-        const uint32_t e = cl[k];
-        const int x = bx + (int)(e & 7u), y = by + (int)((e >> 3) & 7u), z = bz + (int)(e >> 6);
-        sv = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        if (live && (uint32_t)x < dim && (uint32_t)y < dim && (uint32_t)z < dim)
-          sv = __ldg(&src[lvl_base + lin3((uint32_t)x, (uint32_t)y, (uint32_t)z, dim)]);
+      // Children of the neighbour parent at (ox, oy, oz) - 1; null outside the grid.
+      auto block = [&](uint32_t ox, uint32_t oy, uint32_t oz) -> const float4 * {
+        const uint32_t qx = upx + ox - 1u, qy = upy + oy - 1u, qz = upz + oz - 1u;
+        return live && qx < pdim && qy < pdim && qz < pdim ? src + lvl_base + lin3(2u * qx, 2u * qy, 2u * qz, dim) : nullptr;
       };
-      static_assert(kContrib % 2u == 1u, "the loop below ends with one single slot");
+      auto fetch = [&](const float4 *at, float4 &a, float4 &b) {
+        a = b = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (at != nullptr) {
+          a = __ldg(at);
+          b = __ldg(at + 1);
+        }
+      };
+      // The next row's two cells are requested while this row's are evaluated.
+      const float4 *at = block(0u, 0u, 0u);
       float4 n0, n1;
-      fetch(0u, n0);
-      fetch(1u, n1);
-      for (uint32_t k = 0; k + 1u < kContrib; k += 2u) {
-        const float4 s0 = n0, s1 = n1;
-        fetch(k + 2u, n0);  // k + 2 <= kContrib - 1
-        if (k + 3u < kContrib) fetch(k + 3u, n1);
-        // Both 1/r chains first, then the terms slot by slot (absent and
-        // empty slots read w = 0 and add nothing).
-        const PairSetup p0 = pair_setup(s0, ctx, cty, ctz, eps);
-        const PairSetup p1 = pair_setup(s1, ctx, cty, ctz, eps);
-        if (s0.w != 0.0f) {
-          float out[10];
-          pair_terms(p0, out);
-#pragma unroll
-          for (int m = 0; m < 10; m++) acc[m] = acc[m] + out[m];
+      fetch(at, n0, n1);
+      uint32_t ox = 0u, oy = 0u, oz = 0u;
+#pragma unroll 1
+      for (uint32_t b = 0; b < 27u; b++) {
+        uint32_t ex = ox + 1u, ey = oy, ez = oz;  // the next neighbour
+        if (ex == 3u) {
+          ex = 0u;
+          ey++;
         }
-        if (s1.w != 0.0f) {
-          float out[10];
-          pair_terms(p1, out);
-#pragma unroll
-          for (int m = 0; m < 10; m++) acc[m] = acc[m] + out[m];
+        if (ey == 3u) {
+          ey = 0u;
+          ez++;
         }
-      }
-      if (n0.w != 0.0f) {  // the last slot (kContrib - 1)
-        float out[10];
-        pair_field_d(n0, ctx, cty, ctz, eps, out);
+        const float4 *after = b < 26u ? block(ex, ey, ez) : nullptr;
 #pragma unroll
-        for (int m = 0; m < 10; m++) acc[m] = acc[m] + out[m];
+        for (uint32_t row = 0; row < 4u; row++) {
+          float4 s0 = n0, s1 = n1;
+          if (row < 3u)
+            fetch(at == nullptr ? nullptr : at + ((row + 1u) & 1u) * dim + ((row + 1u) >> 1) * dim * dim, n0, n1);
+          else
+            fetch(after, n0, n1);
+          const uint32_t yz = (near_y >> (2u * oy + (row & 1u))) & (near_z >> (2u * oz + (row >> 1)));
+          const uint32_t near = yz & 1u ? near_x >> (2u * ox) : 0u;
+          if (near & 1u) s0.w = 0.0f;
+          if (near & 2u) s1.w = 0.0f;
+          if (s0.w != 0.0f || s1.w != 0.0f)
+            pair_field_two(s0, s1, ctx, cty, ctz, eps, mz,
+                           [&](int k, float u, float v) { acc[k] = (acc[k] + u) + v; });
+        }
+        at = after;
+        ox = ex;
+        oy = ey;
+        oz = ez;
       }
     }
     if (live) {
@@ -829,10 +823,9 @@ __global__ void __launch_bounds__(256, kWide ? 4 : 6) k_m2l(const SceneDesc *__r
                                              const float4 *__restrict__ src,
                                              float *__restrict__ lfield,
                                              const CUtensorMap *__restrict__ tmaps,
-                                             uint32_t lane_min,
+                                             uint32_t lane_min, float minus_zero,
                                              unsigned long long *__restrict__ stamp) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  __shared__ uint16_t s_clist[kWide ? 8 : 1][kContrib];  // the lane path's per-child slot lists
   // The TMA destination must be 128-byte aligned: align the carve-out by hand
   // (the launch reserves 128 spare bytes).
   const uint32_t pad = (128u - (smem_u32(smem_raw) & 127u)) & 127u;
@@ -845,14 +838,13 @@ __global__ void __launch_bounds__(256, kWide ? 4 : 6) k_m2l(const SceneDesc *__r
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   for (uint32_t k = tid; k < kTileCells; k += blockDim.x) sh.slot_info[k] = kStencil.slot[k];
-  if (kWide) copy_child_slots(s_clist);
   grid_dependency_wait();  // the upward pass built the tree and the parent list
   stamp_begin(stamp);
   const uint32_t count = min(ctr->parents[list_par], plist_cap);
   if (blockIdx.x == 0 && tid == 0) ctr->parents[list_par ^ 1u] = 0u;  // reset for the next step
   __syncthreads();
   if (kWide && count >= lane_min) {  // grid-uniform
-    m2l_lanes_pass(scenes, plist, count, mom, src, lfield, s_clist);
+    m2l_lanes_pass(scenes, plist, count, mom, src, lfield, pack2(minus_zero, minus_zero));
     stamp_end(stamp);
     grid_dependents_may_launch();
     return;
@@ -1304,7 +1296,7 @@ void launch_m2l(const LaunchCtx &L, uint32_t list_par) {
   launch_step_kernel(L, kernel, dim3(L.m2l_ctas), dim3(256),
                      m2l_smem_bytes(L.m2l_compact), L.scenes,
                      (const WorkItem *)L.plist, L.plist_cap, L.ctr, list_par, (const uint4 *)L.mom,
-                     (const float4 *)L.src, L.lfield, L.tmaps, lane_min(L.m2l_lanes, kM2LLaneAuto),
+                     (const float4 *)L.src, L.lfield, L.tmaps, lane_min(L.m2l_lanes, kM2LLaneAuto), -0.0f,
                      stamp_rec(L, 1u));
 }
 
@@ -1319,7 +1311,7 @@ void launch_l2l_near(const LaunchCtx &L, uint32_t list_par) {
 cudaError_t configure_tree_kernels() {
   cudaError_t e = cudaSuccess;
   const std::pair<void (*)(const SceneDesc *, const WorkItem *, uint32_t, Counters *, uint32_t,
-                            const uint4 *, const float4 *, float *, const CUtensorMap *, uint32_t,
+                            const uint4 *, const float4 *, float *, const CUtensorMap *, uint32_t, float,
                             unsigned long long *),
                   bool>
       m2l[4] = {{k_m2l<false, false>, false}, {k_m2l<false, true>, false}, {k_m2l<true, false>, true},
