@@ -61,13 +61,11 @@ __device__ __forceinline__ void soft_wall(float &p, float &v, float world_edge, 
 
 // Near-field P2P inputs: the leaf-sorted position snapshot, the per-leaf
 // start table (Morton order, absolute slots, 8^depth + 1 entries per scene at
-// the scene's cell offset), the body's own slot, and (integrate) the pair
-// sums k_near_p2p already formed for every slot, or null: form them here.
+// the scene's cell offset) and the body's own slot.
 struct P2PView {
   const float4 *pos;
   const uint32_t *starts;
   uint32_t self;
-  const float4 *near = nullptr;
 };
 
 // The cell a body samples its field from (wgsl:625-639): the first level
@@ -183,14 +181,7 @@ __device__ __forceinline__ uint32_t body_acceleration(const SceneDesc &S, float 
 
     if (kP2P) {
       float sx, sy, sz, sp = 0.0f;
-      if (!kPhi && V->near != nullptr) {
-        const float4 nr = V->near[V->self];
-        sx = nr.x;
-        sy = nr.y;
-        sz = nr.z;
-      } else {
-        p2p_sums<kPhi>(S, *V, chosen, lx >> csh, ly >> csh, lz >> csh, px, py, pz, sx, sy, sz, sp);
-      }
+      p2p_sums<kPhi>(S, *V, chosen, lx >> csh, ly >> csh, lz >> csh, px, py, pz, sx, sy, sz, sp);
       const float gm = S.gravity / S.n_f;
       ax = ax + gm * sx;
       ay = ay + gm * sy;
@@ -235,23 +226,165 @@ __device__ __forceinline__ uint32_t body_acceleration(const SceneDesc &S, float 
     return count;
 }
 
-// One body's integrate (wgsl:613-771).  Writes the new state into p0/p1 and
-// the new position's leaf cell and fixed-point coordinates (the next deposit).
+// What integrate needs of a scene's descriptor and level constants, worked out
+// once per scene change instead of once per body.
+struct alignas(16) StepScene {
+  float cell_scale;     // 2^(D - 1) / 1.6: leaf cells per unit length
+  float cell_half;      // 2^(D - 1) - 0.5
+  float cell_margin;    // 0.5 - 2^(D - 22)
+  float inner;          // |coordinate| up to which the short deposit path runs
+  uint32_t cell_base;   // index of the scene's leaf (0, 0, 0), less the biased coordinates' bits
+  uint32_t dim, dim2;   // 2^D and 2^(2D)
+  uint32_t cell_off;
+  uint32_t n, body_off;
+  uint32_t level_exp;   // (127 - D) << 23
+  float softening;
+  float dt, gain_up, gain_down;  // dt_eff; clamp(dt * 10, 0, 1) and clamp(dt * 1.05, 0, 1)
+  float scale;          // fixed-point deposit scale
+};
+constexpr float kBias = 0x1.8p23f;  // v + kBias rounds v to an integer, in the sum's low bits
+constexpr uint32_t kBiasBits = 0x4B400000u;
+
+__device__ __forceinline__ StepScene step_scene(const SceneDesc &S) {
+  const float world_edge = kHalf * 0.985f, edge_band = 0.12f * kHalf;
+  const uint32_t D = S.depth;
+  StepScene C;
+  C.cell_scale = __int_as_float(__float_as_int(0.3125f) + (int)(D << 23));  // RN(1 / 3.2) 2^D
+  C.cell_half = __int_as_float((int)(126u + D) << 23) - 0.5f;
+  C.cell_margin = 0.5f - __int_as_float((int)(105u + D) << 23);
+  // Inside the soft wall's band; none with a scale whose fixed-point
+  // coordinates could pass 2^22.
+  C.inner = fabsf(S.scale) <= 0x1p21f ? world_edge - edge_band : -1.0f;
+  C.dim = 1u << D;
+  C.dim2 = 1u << (2u * D);
+  C.cell_base = S.cell_off + level_offset_d(D) - kBiasBits * (1u + C.dim + C.dim2);
+  C.cell_off = S.cell_off;
+  C.n = S.n;
+  C.body_off = S.body_off;
+  C.level_exp = (127u - D) << 23;
+  C.softening = S.softening;
+  C.dt = S.dt_eff;
+  C.gain_up = clampf_d(S.dt_eff * 10.0f, 0.0f, 1.0f);
+  C.gain_down = clampf_d(S.dt_eff * 1.05f, 0.0f, 1.0f);
+  C.scale = S.scale;
+  return C;
+}
+
+// max(|x|, |y|, |z|), NaN if one of them is.
+__device__ __forceinline__ float max_abs3(float x, float y, float z) {
+  float m;
+  asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(m) : "f"(fabsf(x)), "f"(fabsf(y)), "f"(fabsf(z)));
+  return m;
+}
+
+// The leaf a position lies in, as biased coordinates (t - kBias is the cell
+// per axis).  w = p 2^D / 3.2 + 2^(D - 1) - 0.5 by one multiply-add differs
+// from u 2^D - 0.5 (u: unit_coord) by at most 2^(D - 23), as in
+// cells_of_position, so where its distance d from the nearest integer stays
+// below 0.5 - 2^(D - 22) that integer is floor(u 2^D).  False where it is not,
+// and for positions beyond 1.59 (unit_coord clamps above) and NaN.
+__device__ __forceinline__ bool biased_cells(const StepScene &C, float px, float py, float pz, float &tx, float &ty,
+                                             float &tz) {
+  const float wx = __fmaf_rn(px, C.cell_scale, C.cell_half), wy = __fmaf_rn(py, C.cell_scale, C.cell_half),
+              wz = __fmaf_rn(pz, C.cell_scale, C.cell_half);
+  tx = __fadd_rn(wx, kBias);
+  ty = __fadd_rn(wy, kBias);
+  tz = __fadd_rn(wz, kBias);
+  return max_abs3(__fadd_rn(wx, -__fadd_rn(tx, -kBias)), __fadd_rn(wy, -__fadd_rn(ty, -kBias)),
+                  __fadd_rn(wz, -__fadd_rn(tz, -kBias))) <= C.cell_margin;
+}
+__device__ __forceinline__ void biased_cells_slow(const StepScene &C, float px, float py, float pz, float &tx,
+                                                  float &ty, float &tz) {
+  tx = (float)cell_of_unit(unit_coord(px), C.dim) + kBias;
+  ty = (float)cell_of_unit(unit_coord(py), C.dim) + kBias;
+  tz = (float)cell_of_unit(unit_coord(pz), C.dim) + kBias;
+}
+__device__ __forceinline__ uint32_t leaf_index(const StepScene &C, float tx, float ty, float tz) {
+  return __float_as_uint(tz) * C.dim2 + (__float_as_uint(ty) * C.dim + (__float_as_uint(tx) + C.cell_base));
+}
+
+// RN(sqrt(max(x, lo^2))) for lo = 1e-4: max(RN(sqrt(x)), 1e-4), since the root
+// is monotonic and RN(sqrt(RN(lo^2))) = lo.
+__device__ __forceinline__ float length_floor(float x, float y, float z) {
+  const float s = fmaxf((x * x + y * y) + z * z, 0.0001f * 0.0001f);
+#ifdef RFMM_FAST_FLOAT
+  return sqrtf(s);
+#else
+  const float r = sqrt_from_estimate(s, rsqrt_estimate(s));
+  return s < 0x1p127f ? r : sqrtf(s);
+#endif
+}
+
+// One body's integrate (wgsl:613-771): adaptive sample cell, local expansion
+// about its centre, softened self-leaf monopole (kP2P: the pair sums `near`
+// instead), control field, symplectic Euler.  Writes the new state into p0/p1
+// and the new position's leaf cell and fixed-point coordinates plus kBiasBits
+// (the next deposit).
 template <bool kP2P>
-__device__ __forceinline__ void integrate_body(const SceneDesc &S, float4 &p0, float4 &p1,
+__device__ __forceinline__ void integrate_body(const SceneDesc &S, const StepScene &C, float4 &p0, float4 &p1,
                                                const uint4 *__restrict__ mom,
                                                const float4 *__restrict__ src,
                                                const float4 *__restrict__ aux,
                                                const uint32_t *__restrict__ choice,
-                                               const float *__restrict__ fields, uint32_t &key,
-                                               int32_t &qx, int32_t &qy, int32_t &qz,
-                                               const P2PView *V) {
+                                               const float *__restrict__ fields, const float4 *near, uint32_t &key,
+                                               uint32_t &qx, uint32_t &qy, uint32_t &qz) {
     float px = p0.x, py = p0.y, pz = p0.z;
     float vx = p1.x, vy = p1.y, vz = p1.z;
-    const uint32_t D = S.depth;
-    float ax, ay, az, density_pulse;
-    body_acceleration<false, kP2P>(S, px, py, pz, mom, src, aux, choice, fields, ax, ay, az,
-                                   density_pulse, nullptr, V);
+    float tx, ty, tz;
+    if (!biased_cells(C, px, py, pz, tx, ty, tz) || !(max_abs3(px, py, pz) <= 1.59f))
+      biased_cells_slow(C, px, py, pz, tx, ty, tz);
+
+    // The cell the field is sampled from (wgsl:625-639), see sample_cell.
+    const uint32_t pick = __ldg(&choice[leaf_index(C, tx, ty, tz)]);
+    uint32_t e = (pick >> 5) & 0x07800000u;  // its level, in a float's exponent field
+    uint32_t cell = C.cell_off + (pick & 0x0FFFFFFFu);
+    if (pick == kChoiceUnresolved) {
+      uint32_t level, lx, ly, lz;
+      cell = sample_cell(S, px, py, pz, mom, choice, level, lx, ly, lz);
+      e = level << 23;
+    }
+    const float4 ax4 = __ldg(&aux[cell]);
+    const float4 *fp = reinterpret_cast<const float4 *>(fields + (size_t)cell * 12u);
+    const float4 fa = __ldg(fp), fj0 = __ldg(fp + 1), fj1 = __ldg(fp + 2);
+    // Its centre: the leaf coordinate scaled down and rounded down is the
+    // cell's, ((c + 0.5) 2^(1 - l) - 1) kHalf its centre.  The two products
+    // with powers of two are exact, so one rounding each serves.
+    const float down = __uint_as_float(C.level_exp + e), width = __uint_as_float(0x40000000u - e);
+    auto centre = [&](float t) {
+      const float c = __fadd_rn(__fmaf_rd(__fadd_rn(t, -kBias), down, kBias), -kBias);
+      return __fmaf_rn(__fadd_rn(c, 0.5f), width, -1.0f) * kHalf;
+    };
+    const float rx = px - centre(tx), ry = py - centre(ty), rz = pz - centre(tz);
+    float ax = fa.x + (fj0.x * rx + fj0.y * ry + fj0.z * rz);
+    float ay = fa.y + (fj0.y * rx + fj0.w * ry + fj1.x * rz);
+    float az = fa.z + (fj0.z * rx + fj1.x * ry + fj1.y * rz);
+
+    if (kP2P) {
+      const float4 nr = *near;
+      const float gm = S.gravity / S.n_f;
+      ax = ax + gm * nr.x;
+      ay = ay + gm * nr.y;
+      az = az + gm * nr.z;
+    } else if (__float_as_uint(ax4.z) > 1u) {
+      // Self leaf: softened monopole of the other count-1 bodies (wgsl:646-657).
+      const float4 s = __ldg(&src[cell]);
+      const float dx = s.x - px, dy = s.y - py, dz = s.z - pz;
+      const float eps = fmaxf(C.softening, __uint_as_float(__float_as_uint(0.62f * kHalf) - e));
+      const float inv_r = inv_sqrt((dx * dx + dy * dy) + dz * dz + eps * eps);
+      const float gsm = ax4.x;  // G * f32(count - 1) / f32(N)
+#ifdef RFMM_FAST_FLOAT
+      // One weight for the three components (reassociated: fast variant only).
+      const float w = gsm * ((inv_r * inv_r) * inv_r);
+      ax = ax + dx * w;
+      ay = ay + dy * w;
+      az = az + dz * w;
+#else
+      ax = ax + gsm * dx * inv_r * inv_r * inv_r;
+      ay = ay + gsm * dy * inv_r * inv_r * inv_r;
+      az = az + gsm * dz * inv_r * inv_r * inv_r;
+#endif
+    }
+    const float density_pulse = ax4.y;  // clamp((f32(count) - 16) / 72, 0, 1)
 
     // Interactive control field (wgsl:659-689); off unless control_point.w > 0.5.
     float control_influence = 0.0f;
@@ -288,9 +421,7 @@ __device__ __forceinline__ void integrate_body(const SceneDesc &S, float4 &p0, f
     }
 
     // Symplectic Euler with excitation and hue state (wgsl:691-769).
-    const float dt = S.dt_eff;
-    const float radius = fmaxf(length3(px, py, pz), 0.0001f);
-    const float vlen = fmaxf(length3(vx, vy, vz), 0.0001f);
+    const float radius = length_floor(px, py, pz), vlen = length_floor(vx, vy, vz);
     const float pv = (px * vx + py * vy) + pz * vz;
     const float signed_radial = clampf_d(pv / (radius * vlen), -1.0f, 1.0f);
     const float rf = fabsf(signed_radial);
@@ -300,43 +431,49 @@ __device__ __forceinline__ void integrate_body(const SceneDesc &S, float4 &p0, f
                                           field_strength * 0.13f + control_influence * 0.42f,
                                       0.0f, 1.0f);
     float exc = p1.w;
-    const float response = target_exc > exc ? 10.0f : 1.05f;
-    const float t = clampf_d(dt * response, 0.0f, 1.0f);
+    const float t = target_exc > exc ? C.gain_up : C.gain_down;
     exc = exc * (1.0f - t) + target_exc * t;
 
-    vx = vx + ax * dt;
-    vy = vy + ay * dt;
-    vz = vz + az * dt;
-    px = px + vx * dt;
-    py = py + vy * dt;
-    pz = pz + vz * dt;
+    vx = vx + ax * C.dt;
+    vy = vy + ay * C.dt;
+    vz = vz + az * C.dt;
+    px = px + vx * C.dt;
+    py = py + vy * C.dt;
+    pz = pz + vz * C.dt;
 
-    const float world_edge = kHalf * 0.985f;
-    const float edge_band = 0.12f * kHalf;
-    // Inside the band on every axis the walls change nothing (|p| - c > 0 is
-    // |p| > c in binary32 too): one test for the three axes instead of 30
-    // instructions (22.5 -> 21.8 us at 1,048,576 Plummer bodies, 95.5 -> 92.3
-    // at 5,242,880 clustered, 336 -> 324 at 256 scenes).
-    if (fmaxf(fmaxf(fabsf(px), fabsf(py)), fabsf(pz)) > world_edge - edge_band) {
+    // The next step's deposit (wgsl:414-421 on the new position).  Inside the
+    // soft wall's band on every axis the walls change nothing, and adding
+    // kBias rounds the fixed-point coordinates to the nearest even integer.
+    bool inner = max_abs3(px, py, pz) <= C.inner;
+    qx = __float_as_uint(__fadd_rn(px * C.scale, kBias));
+    qy = __float_as_uint(__fadd_rn(py * C.scale, kBias));
+    qz = __float_as_uint(__fadd_rn(pz * C.scale, kBias));
+    inner = biased_cells(C, px, py, pz, tx, ty, tz) && inner;
+    if (!inner) {
+      const float world_edge = kHalf * 0.985f, edge_band = 0.12f * kHalf;
       soft_wall(px, vx, world_edge, edge_band);
       soft_wall(py, vy, world_edge, edge_band);
       soft_wall(pz, vz, world_edge, edge_band);
+      qx = (uint32_t)f2i_rn_sat(px * C.scale) + kBiasBits;
+      qy = (uint32_t)f2i_rn_sat(py * C.scale) + kBiasBits;
+      qz = (uint32_t)f2i_rn_sat(pz * C.scale) + kBiasBits;
+      biased_cells_slow(C, px, py, pz, tx, ty, tz);
     }
+    key = leaf_index(C, tx, ty, tz);
+
+    // Clamped to [0, kWidth] before the division instead of [0, 1] after it
+    // (the quotient is monotonic and kWidth / kWidth = 1), x = 0 or |x| > 2^-27
+    // and finite: the corrected estimate is the rounded quotient.
     constexpr float kWidth = 0.70f - 0.30f, kWidthRcp = 0x1.400002p+1f;  // RN(1 / kWidth)
-    const float st = clampf_d(div_by_const(exc - 0.30f, kWidth, kWidthRcp), 0.0f, 1.0f);
+    const float x = clampf_d(exc - 0.30f, 0.0f, kWidth), q0 = __fmul_rn(x, kWidthRcp);
+    const float st = __fmaf_rn(__fmaf_rn(-q0, kWidth, x), kWidthRcp, q0);
     const float hue_drift = 1.0f - st * st * (3.0f - 2.0f * st);
-    const float hsum = p0.w + dt * hue_drift *
+    const float hsum = p0.w + C.dt * hue_drift *
                                   (0.012f + signed_radial * 0.030f + exc * 0.036f +
                                    control_influence * 0.080f);
     const float hue = hsum - floorf(hsum);
     p0 = make_float4(px, py, pz, hue);
     p1 = make_float4(vx, vy, vz, exc);
-
-    // The next step's deposit (wgsl:414-421 on the new position).
-    key = S.cell_off + leaf_cell(px, py, pz, D);
-    qx = f2i_rn_sat(px * S.scale);
-    qy = f2i_rn_sat(py * S.scale);
-    qz = f2i_rn_sat(pz * S.scale);
 }
 
 // Persistent integrate: CTA c of G walks body tiles c, c + G, c + 2G, ...
@@ -347,18 +484,16 @@ __device__ __forceinline__ void integrate_body(const SceneDesc &S, float4 &p0, f
 //
 // kP2P: near field by exact pair sums over the leaf-sorted position snapshot;
 // no deposit (the end-of-step sort deposits the new positions).
-// Resident CTAs per SM: six in the exact contract (40 registers; 6 / 5 at
-// 1,048,576 Plummer bodies 21.8 / 22.9 us, 5,242,880 clustered 92.3 / 94.8,
-// 256 scenes 324 / 331: more warps cover the per-body dependent chain), five
-// in the fast variant, whose shorter chains gain more from the registers
-// (20.1 / 19.2 and 76.7 / 75.0 us).
-#ifdef RFMM_FAST_FLOAT
-constexpr uint32_t kIntegrateCtas = 5u;
-#else
-constexpr uint32_t kIntegrateCtas = 6u;
-#endif
+// Resident CTAs per SM: five (48 registers; 6 / 5 at 1,048,576 Plummer bodies
+// 20.8 / 20.7 us, uniform 17.2 / 16.2, 5,242,880 clustered 84.3 / 83.5, 256
+// scenes 300 / 295).
+//
+// With the level constants in StepScene, the biased cell coordinates and
+// rounding by kBias, before -> now: 1,048,576 Plummer bodies 21.1 -> 20.7 us,
+// uniform 18.3 -> 16.2, 5,242,880 clustered 90.7 -> 83.5 (fast 73.3 -> 70.2),
+// 256 scenes 321 -> 295 (fast 258 -> 253): what bounds it is instruction issue.
 template <bool kP2P>
-__global__ void __launch_bounds__(256, kIntegrateCtas) k_integrate(const SceneDesc *__restrict__ scenes,
+__global__ void __launch_bounds__(256, 5) k_integrate(const SceneDesc *__restrict__ scenes,
                                                    const uint32_t *__restrict__ tile_scene,
                                                    float4 *__restrict__ part,
                                                    const uint4 *__restrict__ mom,
@@ -369,12 +504,18 @@ __global__ void __launch_bounds__(256, kIntegrateCtas) k_integrate(const SceneDe
                                                    uint4 *__restrict__ mom_next, uint32_t tiles,
                                                    const uint32_t *__restrict__ tile_list,
                                                    Counters *__restrict__ ctr, int dynamic,
-                                                   const float4 *__restrict__ pos4,
-                                                   const uint32_t *__restrict__ starts,
                                                    const float4 *__restrict__ near4,
                                                    unsigned long long *__restrict__ stamp) {
   __shared__ DepositTable T;
   __shared__ SceneDesc S;
+  __shared__ StepScene C;
+  auto enter_scene = [&](uint32_t s) {
+    __syncthreads();
+    if (threadIdx.x < sizeof(SceneDesc) / 4u)
+      reinterpret_cast<uint32_t *>(&S)[threadIdx.x] = reinterpret_cast<const uint32_t *>(scenes + s)[threadIdx.x];
+    if (threadIdx.x == 32u) C = step_scene(scenes[s]);
+    __syncthreads();
+  };
   __shared__ uint32_t s_next;
   if (!kP2P) T.clear();
   // Before the wait for this step's fields: the tile lists and scene
@@ -411,7 +552,7 @@ __global__ void __launch_bounds__(256, kIntegrateCtas) k_integrate(const SceneDe
   if (i < end) {
     load_body(part, next_tile * kTile + threadIdx.x, n0, n1);
     cur = tile_scene[next_tile];
-    load_scene(S, scenes, cur);
+    enter_scene(cur);
   }
   grid_dependency_wait();  // fields of this step are complete
   stamp_begin(stamp);
@@ -431,18 +572,17 @@ __global__ void __launch_bounds__(256, kIntegrateCtas) k_integrate(const SceneDe
     if (ni >= end) grid_dependents_may_launch();
     const uint32_t sc = tile_scene[tile];
     if (sc != cur) {
-      load_scene(S, scenes, sc);
+      enter_scene(sc);
       cur = sc;
     }
-    const bool active = slot - S.body_off < S.n;
+    const bool active = slot - C.body_off < C.n;
     uint32_t key = DepositTable::kEmpty;
-    int32_t qx = 0, qy = 0, qz = 0;
+    uint32_t qx = kBiasBits, qy = kBiasBits, qz = kBiasBits;
     if (active) {
-      const P2PView V{pos4, starts, slot, near4};
-      integrate_body<kP2P>(S, p0, p1, mom, src, aux, choice, fields, key, qx, qy, qz, &V);
+      integrate_body<kP2P>(S, C, p0, p1, mom, src, aux, choice, fields, kP2P ? near4 + slot : nullptr, key, qx, qy, qz);
       store_body(part, slot, p0, p1);
     }
-    if (!kP2P) deposit_body(T, key, active, qx, qy, qz, mom_next);
+    if (!kP2P) deposit_body<kBiasBits>(T, key, active, qx, qy, qz, mom_next);
   }
   if (!kP2P) {
     __syncthreads();
@@ -972,14 +1112,14 @@ __global__ void __launch_bounds__(256) k_deposit(const SceneDesc *__restrict__ s
     }
     const bool active = slot - S.body_off < S.n;
     uint32_t key = DepositTable::kEmpty;
-    int32_t qx = 0, qy = 0, qz = 0;
+    uint32_t qx = 0, qy = 0, qz = 0;
     if (active) {
       key = S.cell_off + leaf_cell(p.x, p.y, p.z, S.depth);
-      qx = f2i_rn_sat(p.x * S.scale);
-      qy = f2i_rn_sat(p.y * S.scale);
-      qz = f2i_rn_sat(p.z * S.scale);
+      qx = (uint32_t)f2i_rn_sat(p.x * S.scale);
+      qy = (uint32_t)f2i_rn_sat(p.y * S.scale);
+      qz = (uint32_t)f2i_rn_sat(p.z * S.scale);
     }
-    deposit_body(T, key, active, qx, qy, qz, moments);
+    deposit_body<0u>(T, key, active, qx, qy, qz, moments);
   }
   __syncthreads();
   T.flush(moments);
@@ -1171,17 +1311,17 @@ __global__ void __launch_bounds__(256) k_gather(const SceneDesc *__restrict__ sc
     }
     const bool active = slot - S.body_off < S.n;
     uint32_t key = DepositTable::kEmpty;
-    int32_t qx = 0, qy = 0, qz = 0;
+    uint32_t qx = 0, qy = 0, qz = 0;
     if (active) {
       store_body(part_out, slot, p0, p1);
       ids_out[slot] = ids_in != nullptr && here < slots ? ids_in[here] : here - S.body_off;
       if (pos_out != nullptr) pos_out[slot] = p0;
       key = S.cell_off + leaf_cell(p0.x, p0.y, p0.z, S.depth);
-      qx = f2i_rn_sat(p0.x * S.scale);
-      qy = f2i_rn_sat(p0.y * S.scale);
-      qz = f2i_rn_sat(p0.z * S.scale);
+      qx = (uint32_t)f2i_rn_sat(p0.x * S.scale);
+      qy = (uint32_t)f2i_rn_sat(p0.y * S.scale);
+      qz = (uint32_t)f2i_rn_sat(p0.z * S.scale);
     }
-    deposit_body(T, key, active, qx, qy, qz, deposit_into);
+    deposit_body<0u>(T, key, active, qx, qy, qz, deposit_into);
   }
   __syncthreads();
   T.flush(deposit_into);
@@ -1362,8 +1502,7 @@ void launch_integrate(const LaunchCtx &L, uint32_t tiles) {
                      dim3(kTile), 0, L.scenes, L.tile_scene, L.part, (const uint4 *)L.mom,
                      (const float4 *)L.src, (const float4 *)L.aux, (const uint32_t *)L.choice,
                      (const float *)L.fields, L.mom_next, tiles, L.tile_list, L.ctr,
-                     L.integrate_dynamic ? 1 : 0, L.pos4, (const uint32_t *)L.starts_out,
-                     (const float4 *)L.near4, stamp_rec(L, 3u));
+                     L.integrate_dynamic ? 1 : 0, (const float4 *)L.near4, stamp_rec(L, 3u));
 }
 
 // One wave of the pair-sum kernel's resident CTAs, at most one warp per unit.
