@@ -1308,6 +1308,8 @@ void launch_l2l_near(const LaunchCtx &L, uint32_t list_par) {
                      lane_min(L.l2l_lanes, kL2LLaneAuto), stamp_rec(L, 2u));
 }
 
+constexpr int kUpwardCarveout = 58;  // percent of the SM's shared memory: 132 KB
+
 cudaError_t configure_tree_kernels() {
   cudaError_t e = cudaSuccess;
   const std::pair<void (*)(const SceneDesc *, const WorkItem *, uint32_t, Counters *, uint32_t,
@@ -1320,6 +1322,15 @@ cudaError_t configure_tree_kernels() {
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(k.first, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)m2l_smem_bytes(k.second));
+  // The upward pass starts on SMs that integrate is leaving.  With the
+  // driver's choice (hardly any shared memory) between the many-scene launches'
+  // larger ones, every such SM has to empty before its memory is divided
+  // anew, around each early launch: 256 scenes, 20 steps, 14.9 ms with 132 KB,
+  // 15.0 with 164 KB, 16.3 to 17.2 with the driver's choice.  (One scene: no
+  // difference.  The same setting for integrate costs the 5,242,880-body
+  // step 1 % of L1.)
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(k_upward<true>, cudaFuncAttributePreferredSharedMemoryCarveout, kUpwardCarveout);
   return e;
 }
 
