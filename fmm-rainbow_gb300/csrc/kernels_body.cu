@@ -15,6 +15,8 @@
 // the tree gathers broadcast and the deposit is one reduction per run.
 #include <cuda_runtime.h>
 
+#include <type_traits>
+
 #include "rfmm_device.cuh"
 #include "rfmm_kernels.h"
 #include "rfmm_math.h"
@@ -277,203 +279,321 @@ __device__ __forceinline__ float max_abs3(float x, float y, float z) {
   return m;
 }
 
-// The leaf a position lies in, as biased coordinates (t - kBias is the cell
+// The leaves positions lie in, as biased coordinates (t - kBias is the cell
 // per axis).  w = p 2^D / 3.2 + 2^(D - 1) - 0.5 by one multiply-add differs
 // from u 2^D - 0.5 (u: unit_coord) by at most 2^(D - 23), as in
 // cells_of_position, so where its distance d from the nearest integer stays
-// below 0.5 - 2^(D - 22) that integer is floor(u 2^D).  False where it is not,
-// and for positions beyond 1.59 (unit_coord clamps above) and NaN.
-__device__ __forceinline__ bool biased_cells(const StepScene &C, float px, float py, float pz, float &tx, float &ty,
-                                             float &tz) {
-  const float wx = __fmaf_rn(px, C.cell_scale, C.cell_half), wy = __fmaf_rn(py, C.cell_scale, C.cell_half),
-              wz = __fmaf_rn(pz, C.cell_scale, C.cell_half);
-  tx = __fadd_rn(wx, kBias);
-  ty = __fadd_rn(wy, kBias);
-  tz = __fadd_rn(wz, kBias);
-  return max_abs3(__fadd_rn(wx, -__fadd_rn(tx, -kBias)), __fadd_rn(wy, -__fadd_rn(ty, -kBias)),
-                  __fadd_rn(wz, -__fadd_rn(tz, -kBias))) <= C.cell_margin;
+// below 0.5 - 2^(D - 22) that integer is floor(u 2^D).  ok: whether it does on
+// every axis.
+template <class V, int kN>
+__device__ __forceinline__ void biased_cells(const StepScene &C, const V (&p)[3], V (&t)[3], bool (&ok)[kN]) {
+  V scale, half, bias, unbias;
+  splat(scale, C.cell_scale);
+  splat(half, C.cell_half);
+  splat(bias, kBias);
+  splat(unbias, -kBias);
+  float d[3][kN];
+#pragma unroll
+  for (int c = 0; c < 3; c++) {
+    const V w = fma2(p[c], scale, half);
+    t[c] = add2(w, bias);
+    halves(sub2(w, add2(t[c], unbias)), d[c]);
+  }
+#pragma unroll
+  for (int h = 0; h < kN; h++) ok[h] = max_abs3(d[0][h], d[1][h], d[2][h]) <= C.cell_margin;
 }
-__device__ __forceinline__ void biased_cells_slow(const StepScene &C, float px, float py, float pz, float &tx,
-                                                  float &ty, float &tz) {
-  tx = (float)cell_of_unit(unit_coord(px), C.dim) + kBias;
-  ty = (float)cell_of_unit(unit_coord(py), C.dim) + kBias;
-  tz = (float)cell_of_unit(unit_coord(pz), C.dim) + kBias;
+__device__ __forceinline__ float biased_cell_slow(const StepScene &C, float p) {
+  return (float)cell_of_unit(unit_coord(p), C.dim) + kBias;
 }
 __device__ __forceinline__ uint32_t leaf_index(const StepScene &C, float tx, float ty, float tz) {
   return __float_as_uint(tz) * C.dim2 + (__float_as_uint(ty) * C.dim + (__float_as_uint(tx) + C.cell_base));
 }
 
-// RN(sqrt(max(x, lo^2))) for lo = 1e-4: max(RN(sqrt(x)), 1e-4), since the root
-// is monotonic and RN(sqrt(RN(lo^2))) = lo.
-__device__ __forceinline__ float length_floor(float x, float y, float z) {
-  const float s = fmaxf((x * x + y * y) + z * z, 0.0001f * 0.0001f);
-#ifdef RFMM_FAST_FLOAT
-  return sqrtf(s);
-#else
-  const float r = sqrt_from_estimate(s, rsqrt_estimate(s));
-  return s < 0x1p127f ? r : sqrtf(s);
-#endif
+// Interactive control field (wgsl:659-689): its influence at a position, and
+// its acceleration added to a.
+__device__ __forceinline__ float control_force(const SceneDesc &S, float px, float py, float pz, float &ax, float &ay,
+                                               float &az) {
+  const float cdx = S.control_point[0] - px, cdy = S.control_point[1] - py,
+              cdz = S.control_point[2] - pz;
+  const float d2 = (cdx * cdx + cdy * cdy) + cdz * cdz;
+  const float cr = fmaxf(S.control_radius, 0.02f);
+  const float control_influence = rf_expf(-2.0f * d2 / (cr * cr));
+  const float strength = S.control_strength;
+  const float inv = inv_sqrt(d2 + cr * cr * 0.018f);
+  const float dirx = cdx * inv, diry = cdy * inv, dirz = cdz * inv;
+  const float mode = S.control_axis_mode[3];
+  if (mode < 1.5f) {
+    ax = ax + dirx * strength * control_influence;
+    ay = ay + diry * strength * control_influence;
+    az = az + dirz * strength * control_influence;
+  } else if (mode < 2.5f) {
+    ax = ax - dirx * strength * control_influence;
+    ay = ay - diry * strength * control_influence;
+    az = az - dirz * strength * control_influence;
+  } else {
+    const float al = length3(S.control_axis_mode[0], S.control_axis_mode[1], S.control_axis_mode[2]);
+    const float nx = S.control_axis_mode[0] / al, ny = S.control_axis_mode[1] / al,
+                nz = S.control_axis_mode[2] / al;
+    const float tx = ny * cdz - nz * cdy, ty = nz * cdx - nx * cdz, tz = nx * cdy - ny * cdx;
+    const float tl = length3(tx, ty, tz);
+    if (tl > 0.00001f) {
+      ax = ax + tx / tl * strength * control_influence;
+      ay = ay + ty / tl * strength * control_influence;
+      az = az + tz / tl * strength * control_influence;
+    }
+  }
+  return control_influence;
 }
 
-// One body's integrate (wgsl:613-771): adaptive sample cell, local expansion
-// about its centre, softened self-leaf monopole (kP2P: the pair sums `near`
-// instead), control field, symplectic Euler.  Writes the new state into p0/p1
-// and the new position's leaf cell and fixed-point coordinates plus kBiasBits
-// (the next deposit).
-template <bool kP2P>
-__device__ __forceinline__ void integrate_body(const SceneDesc &S, const StepScene &C, float4 &p0, float4 &p1,
-                                               const uint4 *__restrict__ mom,
-                                               const float4 *__restrict__ src,
-                                               const float4 *__restrict__ aux,
-                                               const uint32_t *__restrict__ choice,
-                                               const float *__restrict__ fields, const float4 *near, uint32_t &key,
-                                               uint32_t &qx, uint32_t &qy, uint32_t &qz) {
-    float px = p0.x, py = p0.y, pz = p0.z;
-    float vx = p1.x, vy = p1.y, vz = p1.z;
-    float tx, ty, tz;
-    if (!biased_cells(C, px, py, pz, tx, ty, tz) || !(max_abs3(px, py, pz) <= 1.59f))
-      biased_cells_slow(C, px, py, pz, tx, ty, tz);
+// Walls, biased cells and fixed-point coordinates of a body for which the
+// short path does not hold.
+__device__ __forceinline__ void outer_deposit(const StepScene &C, float4 &p0, float4 &p1, float &tx, float &ty,
+                                              float &tz, uint32_t (&q)[3]) {
+  const float world_edge = kHalf * 0.985f, edge_band = 0.12f * kHalf;
+  soft_wall(p0.x, p1.x, world_edge, edge_band);
+  soft_wall(p0.y, p1.y, world_edge, edge_band);
+  soft_wall(p0.z, p1.z, world_edge, edge_band);
+  q[0] = (uint32_t)f2i_rn_sat(p0.x * C.scale) + kBiasBits;
+  q[1] = (uint32_t)f2i_rn_sat(p0.y * C.scale) + kBiasBits;
+  q[2] = (uint32_t)f2i_rn_sat(p0.z * C.scale) + kBiasBits;
+  tx = biased_cell_slow(C, p0.x);
+  ty = biased_cell_slow(C, p0.y);
+  tz = biased_cell_slow(C, p0.z);
+}
 
-    // The cell the field is sampled from (wgsl:625-639), see sample_cell.
-    const uint32_t pick = __ldg(&choice[leaf_index(C, tx, ty, tz)]);
-    uint32_t e = (pick >> 5) & 0x07800000u;  // its level, in a float's exponent field
-    uint32_t cell = C.cell_off + (pick & 0x0FFFFFFFu);
-    if (pick == kChoiceUnresolved) {
+// The integrate (wgsl:613-771) of a lane's kN bodies, V holding one value of
+// each: adaptive sample cells, local expansions about their centres, softened
+// self-leaf monopoles (kP2P: the pair sums `near` instead), control field,
+// symplectic Euler.  Writes the new states into lo, hi and the new positions'
+// leaf cells and fixed-point coordinates plus kBiasBits (the next deposit).
+template <bool kP2P, class V, int kN>
+__device__ __forceinline__ void integrate_bodies(const SceneDesc &S, const StepScene &C, V mz, float4 (&lo)[kN],
+                                                 float4 (&hi)[kN], const uint4 *__restrict__ mom,
+                                                 const float4 *__restrict__ src, const float4 *__restrict__ aux,
+                                                 const uint32_t *__restrict__ choice,
+                                                 const float *__restrict__ fields, const float4 *near,
+                                                 uint32_t (&key)[kN], uint32_t (&q)[kN][3]) {
+  auto mul = [&](V x, V y) { return mul2(x, y, mz); };
+  auto all = [](float c) {
+    V v;
+    splat(v, c);
+    return v;
+  };
+  auto per = [](auto &&f) {  // f(h) of every body h
+    float v[kN];
+#pragma unroll
+    for (int h = 0; h < kN; h++) v[h] = f(h);
+    return joined(v);
+  };
+  auto sum_sq = [&](const V (&x)[3]) { return add2(add2(mul(x[0], x[0]), mul(x[1], x[1])), mul(x[2], x[2])); };
+
+  V p[3] = {per([&](int h) { return lo[h].x; }), per([&](int h) { return lo[h].y; }),
+            per([&](int h) { return lo[h].z; })};
+  V t[3];
+  bool ok[kN], every = true;
+  biased_cells(C, p, t, ok);
+#pragma unroll
+  for (int h = 0; h < kN; h++)  // (unit_coord clamps above 1.59)
+    every = every && ok[h] && max_abs3(lo[h].x, lo[h].y, lo[h].z) <= 1.59f;
+  if (!every) {
+    t[0] = per([&](int h) { return biased_cell_slow(C, lo[h].x); });
+    t[1] = per([&](int h) { return biased_cell_slow(C, lo[h].y); });
+    t[2] = per([&](int h) { return biased_cell_slow(C, lo[h].z); });
+  }
+  float u[3][kN];
+#pragma unroll
+  for (int c = 0; c < 3; c++) halves(t[c], u[c]);
+
+  // The cells the fields are sampled from (wgsl:625-639), see sample_cell;
+  // e: their levels, in a float's exponent field.
+  uint32_t pick[kN], e[kN], cell[kN];
+  bool resolved = true;
+#pragma unroll
+  for (int h = 0; h < kN; h++) pick[h] = __ldg(&choice[leaf_index(C, u[0][h], u[1][h], u[2][h])]);
+#pragma unroll
+  for (int h = 0; h < kN; h++) {
+    e[h] = (pick[h] >> 5) & 0x07800000u;
+    cell[h] = C.cell_off + (pick[h] & 0x0FFFFFFFu);
+    resolved = resolved && pick[h] != kChoiceUnresolved;
+  }
+  if (!resolved) {
+#pragma unroll
+    for (int h = 0; h < kN; h++) {
       uint32_t level, lx, ly, lz;
-      cell = sample_cell(S, px, py, pz, mom, choice, level, lx, ly, lz);
-      e = level << 23;
+      cell[h] = sample_cell(S, lo[h].x, lo[h].y, lo[h].z, mom, choice, level, lx, ly, lz);
+      e[h] = level << 23;
     }
-    const float4 ax4 = __ldg(&aux[cell]);
-    const float4 *fp = reinterpret_cast<const float4 *>(fields + (size_t)cell * 12u);
-    const float4 fa = __ldg(fp), fj0 = __ldg(fp + 1), fj1 = __ldg(fp + 2);
-    // Its centre: the leaf coordinate scaled down and rounded down is the
-    // cell's, ((c + 0.5) 2^(1 - l) - 1) kHalf its centre.  The two products
-    // with powers of two are exact, so one rounding each serves.
-    const float down = __uint_as_float(C.level_exp + e), width = __uint_as_float(0x40000000u - e);
-    auto centre = [&](float t) {
-      const float c = __fadd_rn(__fmaf_rd(__fadd_rn(t, -kBias), down, kBias), -kBias);
-      return __fmaf_rn(__fadd_rn(c, 0.5f), width, -1.0f) * kHalf;
-    };
-    const float rx = px - centre(tx), ry = py - centre(ty), rz = pz - centre(tz);
-    float ax = fa.x + (fj0.x * rx + fj0.y * ry + fj0.z * rz);
-    float ay = fa.y + (fj0.y * rx + fj0.w * ry + fj1.x * rz);
-    float az = fa.z + (fj0.z * rx + fj1.x * ry + fj1.y * rz);
+  }
+  float4 x[kN], f[kN], j[kN], k[kN];
+#pragma unroll
+  for (int h = 0; h < kN; h++) {
+    x[h] = __ldg(&aux[cell[h]]);
+    const float4 *fp = reinterpret_cast<const float4 *>(fields + (size_t)cell[h] * 12u);
+    f[h] = __ldg(fp);
+    j[h] = __ldg(fp + 1);
+    k[h] = __ldg(fp + 2);
+  }
+  // Their centres, negated: the leaf coordinate scaled down and rounded down
+  // is the cell's, ((c + 0.5) 2^(1 - l) - 1) kHalf its centre.  The two
+  // products with powers of two are exact, so one rounding each serves.
+  V r[3];
+  {
+    const V down = per([&](int h) { return __uint_as_float(C.level_exp + e[h]); });
+    const V width = per([&](int h) { return __uint_as_float(0x40000000u - e[h]); });
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      const V at = add2(fma2_down(add2(t[c], all(-kBias)), down, all(kBias)), all(-kBias));
+      r[c] = add2(p[c], mul(fma2(add2(at, all(0.5f)), width, all(-1.0f)), all(-kHalf)));
+    }
+  }
+  V a[3];
+  {
+    const V xx = per([&](int h) { return j[h].x; }), xy = per([&](int h) { return j[h].y; }),
+            xz = per([&](int h) { return j[h].z; }), yy = per([&](int h) { return j[h].w; }),
+            yz = per([&](int h) { return k[h].x; }), zz = per([&](int h) { return k[h].y; });
+    auto dot = [&](V g, V tx, V ty, V tz) { return add2(g, add2(add2(mul(tx, r[0]), mul(ty, r[1])), mul(tz, r[2]))); };
+    a[0] = dot(per([&](int h) { return f[h].x; }), xx, xy, xz);
+    a[1] = dot(per([&](int h) { return f[h].y; }), xy, yy, yz);
+    a[2] = dot(per([&](int h) { return f[h].z; }), xz, yz, zz);
+  }
 
-    if (kP2P) {
-      const float4 nr = *near;
-      const float gm = S.gravity / S.n_f;
-      ax = ax + gm * nr.x;
-      ay = ay + gm * nr.y;
-      az = az + gm * nr.z;
-    } else if (__float_as_uint(ax4.z) > 1u) {
-      // Self leaf: softened monopole of the other count-1 bodies (wgsl:646-657).
-      const float4 s = __ldg(&src[cell]);
-      const float dx = s.x - px, dy = s.y - py, dz = s.z - pz;
-      const float eps = fmaxf(C.softening, __uint_as_float(__float_as_uint(0.62f * kHalf) - e));
-      const float inv_r = inv_sqrt((dx * dx + dy * dy) + dz * dz + eps * eps);
-      const float gsm = ax4.x;  // G * f32(count - 1) / f32(N)
+  if (kP2P) {
+    const V gm = all(S.gravity / S.n_f);
+    a[0] = add2(a[0], mul(gm, per([&](int h) { return near[h].x; })));
+    a[1] = add2(a[1], mul(gm, per([&](int h) { return near[h].y; })));
+    a[2] = add2(a[2], mul(gm, per([&](int h) { return near[h].z; })));
+  } else {
+    // Self leaf: softened monopole of the other count-1 bodies (wgsl:646-657).
+    bool any = false, others[kN];
+#pragma unroll
+    for (int h = 0; h < kN; h++) {
+      others[h] = __float_as_uint(x[h].z) > 1u;
+      any = any || others[h];
+    }
+    if (any) {
+      float4 s[kN];
+#pragma unroll
+      for (int h = 0; h < kN; h++) s[h] = __ldg(&src[cell[h]]);
+      const V d[3] = {sub2(per([&](int h) { return s[h].x; }), p[0]), sub2(per([&](int h) { return s[h].y; }), p[1]),
+                      sub2(per([&](int h) { return s[h].z; }), p[2])};
+      const V eps = per([&](int h) { return fmaxf(C.softening, __uint_as_float(__float_as_uint(0.62f * kHalf) - e[h])); });
+      const V inv = inv_sqrt2(add2(sum_sq(d), mul(eps, eps)), mz);
+      const V gsm = per([&](int h) { return x[h].x; });  // G * f32(count - 1) / f32(N)
 #ifdef RFMM_FAST_FLOAT
-      // One weight for the three components (reassociated: fast variant only).
-      const float w = gsm * ((inv_r * inv_r) * inv_r);
-      ax = ax + dx * w;
-      ay = ay + dy * w;
-      az = az + dz * w;
-#else
-      ax = ax + gsm * dx * inv_r * inv_r * inv_r;
-      ay = ay + gsm * dy * inv_r * inv_r * inv_r;
-      az = az + gsm * dz * inv_r * inv_r * inv_r;
+      const V w = mul(gsm, mul(mul(inv, inv), inv));  // one weight (reassociated: fast variant only)
 #endif
-    }
-    const float density_pulse = ax4.y;  // clamp((f32(count) - 16) / 72, 0, 1)
-
-    // Interactive control field (wgsl:659-689); off unless control_point.w > 0.5.
-    float control_influence = 0.0f;
-    if (S.control_point[3] > 0.5f) {
-      const float cdx = S.control_point[0] - px, cdy = S.control_point[1] - py,
-                  cdz = S.control_point[2] - pz;
-      const float d2 = (cdx * cdx + cdy * cdy) + cdz * cdz;
-      const float cr = fmaxf(S.control_radius, 0.02f);
-      control_influence = rf_expf(-2.0f * d2 / (cr * cr));
-      const float strength = S.control_strength;
-      const float inv = inv_sqrt(d2 + cr * cr * 0.018f);
-      const float dirx = cdx * inv, diry = cdy * inv, dirz = cdz * inv;
-      const float mode = S.control_axis_mode[3];
-      if (mode < 1.5f) {
-        ax = ax + dirx * strength * control_influence;
-        ay = ay + diry * strength * control_influence;
-        az = az + dirz * strength * control_influence;
-      } else if (mode < 2.5f) {
-        ax = ax - dirx * strength * control_influence;
-        ay = ay - diry * strength * control_influence;
-        az = az - dirz * strength * control_influence;
-      } else {
-        const float al = length3(S.control_axis_mode[0], S.control_axis_mode[1], S.control_axis_mode[2]);
-        const float nx = S.control_axis_mode[0] / al, ny = S.control_axis_mode[1] / al,
-                    nz = S.control_axis_mode[2] / al;
-        const float tx = ny * cdz - nz * cdy, ty = nz * cdx - nx * cdz, tz = nx * cdy - ny * cdx;
-        const float tl = length3(tx, ty, tz);
-        if (tl > 0.00001f) {
-          ax = ax + tx / tl * strength * control_influence;
-          ay = ay + ty / tl * strength * control_influence;
-          az = az + tz / tl * strength * control_influence;
-        }
+#pragma unroll
+      for (int c = 0; c < 3; c++) {
+#ifdef RFMM_FAST_FLOAT
+        const V with = add2(a[c], mul(d[c], w));
+#else
+        const V with = add2(a[c], mul(mul(mul(mul(gsm, d[c]), inv), inv), inv));
+#endif
+        float without[kN], sum[kN];
+        halves(a[c], without);
+        halves(with, sum);
+        a[c] = per([&](int h) { return others[h] ? sum[h] : without[h]; });
       }
     }
+  }
 
-    // Symplectic Euler with excitation and hue state (wgsl:691-769).
-    const float radius = length_floor(px, py, pz), vlen = length_floor(vx, vy, vz);
-    const float pv = (px * vx + py * vy) + pz * vz;
-    const float signed_radial = clampf_d(pv / (radius * vlen), -1.0f, 1.0f);
-    const float rf = fabsf(signed_radial);
-    const float radial_shock = rf * rf * rf;
-    const float field_strength = clampf_d(length3(ax, ay, az) * (radius + 0.12f) * 0.58f, 0.0f, 1.0f);
-    const float target_exc = clampf_d(0.025f + radial_shock * 0.56f + density_pulse * 0.26f +
-                                          field_strength * 0.13f + control_influence * 0.42f,
-                                      0.0f, 1.0f);
-    float exc = p1.w;
-    const float t = target_exc > exc ? C.gain_up : C.gain_down;
-    exc = exc * (1.0f - t) + target_exc * t;
+  V influence = all(0.0f);
+  if (S.control_point[3] > 0.5f) {
+    float g[3][kN];
+#pragma unroll
+    for (int c = 0; c < 3; c++) halves(a[c], g[c]);
+    influence = per([&](int h) { return control_force(S, lo[h].x, lo[h].y, lo[h].z, g[0][h], g[1][h], g[2][h]); });
+#pragma unroll
+    for (int c = 0; c < 3; c++) a[c] = joined(g[c]);
+  }
 
-    vx = vx + ax * C.dt;
-    vy = vy + ay * C.dt;
-    vz = vz + az * C.dt;
-    px = px + vx * C.dt;
-    py = py + vy * C.dt;
-    pz = pz + vz * C.dt;
+  // Symplectic Euler with excitation and hue state (wgsl:691-769).
+  auto clamped = [&](V v, float low, float high) {
+    float w[kN];
+    halves(v, w);
+    return per([&](int h) { return clampf_d(w[h], low, high); });
+  };
+  // max(RN(sqrt(v)), 1e-4) is the root of max(v, RN(1e-4^2)): the root is
+  // monotonic and RN(sqrt(RN(1e-4^2))) = 1e-4.
+  auto length_floor = [&](V v) {
+    float w[kN];
+    halves(v, w);
+    return sqrt2<true>(per([&](int h) { return fmaxf(w[h], 0.0001f * 0.0001f); }), mz);
+  };
+  V v[3] = {per([&](int h) { return hi[h].x; }), per([&](int h) { return hi[h].y; }),
+            per([&](int h) { return hi[h].z; })};
+  const V radius = length_floor(sum_sq(p)), speed = length_floor(sum_sq(v));
+  float pv[kN], rv[kN];
+  halves(add2(add2(mul(p[0], v[0]), mul(p[1], v[1])), mul(p[2], v[2])), pv);
+  halves(mul(radius, speed), rv);
+  float sr[kN];
+#pragma unroll
+  for (int h = 0; h < kN; h++) sr[h] = clampf_d(pv[h] / rv[h], -1.0f, 1.0f);
+  const V signed_radial = joined(sr), rf = per([&](int h) { return fabsf(sr[h]); });
+  const V strength =
+      clamped(mul(mul(sqrt2<false>(sum_sq(a), mz), add2(radius, all(0.12f))), all(0.58f)), 0.0f, 1.0f);
+  const V pulse = per([&](int h) { return x[h].y; });  // clamp((f32(count) - 16) / 72, 0, 1)
+  const V target = clamped(add2(add2(add2(add2(all(0.025f), mul(mul(mul(rf, rf), rf), all(0.56f))),
+                                          mul(pulse, all(0.26f))),
+                                     mul(strength, all(0.13f))),
+                                mul(influence, all(0.42f))),
+                           0.0f, 1.0f);
+  float goal[kN];
+  halves(target, goal);
+  const V gain = per([&](int h) { return goal[h] > hi[h].w ? C.gain_up : C.gain_down; });
+  const V exc = add2(mul(per([&](int h) { return hi[h].w; }), sub2(all(1.0f), gain)), mul(target, gain));
 
-    // The next step's deposit (wgsl:414-421 on the new position).  Inside the
-    // soft wall's band on every axis the walls change nothing, and adding
-    // kBias rounds the fixed-point coordinates to the nearest even integer.
-    bool inner = max_abs3(px, py, pz) <= C.inner;
-    qx = __float_as_uint(__fadd_rn(px * C.scale, kBias));
-    qy = __float_as_uint(__fadd_rn(py * C.scale, kBias));
-    qz = __float_as_uint(__fadd_rn(pz * C.scale, kBias));
-    inner = biased_cells(C, px, py, pz, tx, ty, tz) && inner;
-    if (!inner) {
-      const float world_edge = kHalf * 0.985f, edge_band = 0.12f * kHalf;
-      soft_wall(px, vx, world_edge, edge_band);
-      soft_wall(py, vy, world_edge, edge_band);
-      soft_wall(pz, vz, world_edge, edge_band);
-      qx = (uint32_t)f2i_rn_sat(px * C.scale) + kBiasBits;
-      qy = (uint32_t)f2i_rn_sat(py * C.scale) + kBiasBits;
-      qz = (uint32_t)f2i_rn_sat(pz * C.scale) + kBiasBits;
-      biased_cells_slow(C, px, py, pz, tx, ty, tz);
+  const V dt = all(C.dt);
+#pragma unroll
+  for (int c = 0; c < 3; c++) {
+    v[c] = add2(v[c], mul(a[c], dt));
+    p[c] = add2(p[c], mul(v[c], dt));
+  }
+  // Clamped to [0, kWidth] before the division instead of [0, 1] after it
+  // (the quotient is monotonic and kWidth / kWidth = 1), n = 0 or |n| > 2^-27
+  // and finite: the corrected estimate is the rounded quotient.
+  constexpr float kWidth = 0.70f - 0.30f, kWidthRcp = 0x1.400002p+1f;  // RN(1 / kWidth)
+  const V n = clamped(add2(exc, all(-0.30f)), 0.0f, kWidth), quot = mul(n, all(kWidthRcp));
+  const V st = fma2(fma2(quot, all(-kWidth), n), all(kWidthRcp), quot);
+  const V drift = sub2(all(1.0f), mul(mul(st, st), sub2(all(3.0f), mul(all(2.0f), st))));
+  const V hue = add2(per([&](int h) { return lo[h].w; }),
+                     mul(mul(dt, drift), add2(add2(add2(all(0.012f), mul(signed_radial, all(0.030f))),
+                                                   mul(exc, all(0.036f))),
+                                              mul(influence, all(0.080f)))));
+  {
+    float o[8][kN];
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      halves(p[c], o[c]);
+      halves(v[c], o[4 + c]);
     }
-    key = leaf_index(C, tx, ty, tz);
+    halves(hue, o[3]);
+    halves(exc, o[7]);
+#pragma unroll
+    for (int h = 0; h < kN; h++) {
+      lo[h] = make_float4(o[0][h], o[1][h], o[2][h], o[3][h] - floorf(o[3][h]));
+      hi[h] = make_float4(o[4][h], o[5][h], o[6][h], o[7][h]);
+    }
+  }
 
-    // Clamped to [0, kWidth] before the division instead of [0, 1] after it
-    // (the quotient is monotonic and kWidth / kWidth = 1), x = 0 or |x| > 2^-27
-    // and finite: the corrected estimate is the rounded quotient.
-    constexpr float kWidth = 0.70f - 0.30f, kWidthRcp = 0x1.400002p+1f;  // RN(1 / kWidth)
-    const float x = clampf_d(exc - 0.30f, 0.0f, kWidth), q0 = __fmul_rn(x, kWidthRcp);
-    const float st = __fmaf_rn(__fmaf_rn(-q0, kWidth, x), kWidthRcp, q0);
-    const float hue_drift = 1.0f - st * st * (3.0f - 2.0f * st);
-    const float hsum = p0.w + C.dt * hue_drift *
-                                  (0.012f + signed_radial * 0.030f + exc * 0.036f +
-                                   control_influence * 0.080f);
-    const float hue = hsum - floorf(hsum);
-    p0 = make_float4(px, py, pz, hue);
-    p1 = make_float4(vx, vy, vz, exc);
+  // The next step's deposit (wgsl:414-421 on the new position).  Inside the
+  // soft wall's band on every axis the walls change nothing, and adding
+  // kBias rounds the fixed-point coordinates to the nearest even integer.
+  biased_cells(C, p, t, ok);
+  float b[3][kN];
+#pragma unroll
+  for (int c = 0; c < 3; c++) {
+    halves(t[c], u[c]);
+    halves(add2(mul(p[c], all(C.scale)), all(kBias)), b[c]);
+  }
+#pragma unroll
+  for (int h = 0; h < kN; h++) {
+#pragma unroll
+    for (int c = 0; c < 3; c++) q[h][c] = __float_as_uint(b[c][h]);
+    if (!(ok[h] && max_abs3(lo[h].x, lo[h].y, lo[h].z) <= C.inner))
+      outer_deposit(C, lo[h], hi[h], u[0][h], u[1][h], u[2][h], q[h]);
+    key[h] = leaf_index(C, u[0][h], u[1][h], u[2][h]);
+  }
 }
 
 // Persistent integrate: CTA c of G walks body tiles c, c + G, c + 2G, ...
@@ -484,16 +604,28 @@ __device__ __forceinline__ void integrate_body(const SceneDesc &S, const StepSce
 //
 // kP2P: near field by exact pair sums over the leaf-sorted position snapshot;
 // no deposit (the end-of-step sort deposits the new positions).
-// Resident CTAs per SM: five (48 registers; 6 / 5 at 1,048,576 Plummer bodies
-// 20.8 / 20.7 us, uniform 17.2 / 16.2, 5,242,880 clustered 84.3 / 83.5, 256
-// scenes 300 / 295).
+// One body per lane, a tile per CTA of 256: with the level constants in
+// StepScene, biased cells and rounding by kBias, 510 instead of 585
+// instructions per 32 bodies (1,048,576 Plummer bodies 21.1 -> 20.7 us,
+// uniform 18.3 -> 16.2, 5,242,880 clustered 90.7 -> 83.5, fast 73.3 -> 70.2,
+// 256 scenes 321 -> 295), still bound by instruction issue.  Two packed bodies
+// per lane, a tile per CTA of 128: 344 instructions, one run scan for both;
+// what bounds it is the latency of six warps per sub-partition (issue active
+// 63 %).  One / two, exact: 250,000 Plummer bodies 6.1 / 8.6, 524,288 11.7 /
+// 12.2 (uniform 9.45 / 9.15), 700,000 13.4 / 13.4, 1,048,576 20.4 / 18.9
+// (uniform 16.2 / 15.4), 5,242,880 clustered 83.3 / 76.6, 256 scenes 295 /
+// 279: pairs pay from about 16 tiles per SM.  The fast variant's contracted
+// chains are shorter and gain nothing from packing (clustered 71 / 73).
 //
-// With the level constants in StepScene, the biased cell coordinates and
-// rounding by kBias, before -> now: 1,048,576 Plummer bodies 21.1 -> 20.7 us,
-// uniform 18.3 -> 16.2, 5,242,880 clustered 90.7 -> 83.5 (fast 73.3 -> 70.2),
-// 256 scenes 321 -> 295 (fast 258 -> 253): what bounds it is instruction issue.
-template <bool kP2P>
-__global__ void __launch_bounds__(256, 5) k_integrate(const SceneDesc *__restrict__ scenes,
+// Resident CTAs per SM: five of 256 (6 / 5: clustered 84.3 / 83.5, 256 scenes
+// 300 / 295), six of 128 (5 / 6 / 7: Plummer 21.9 / 19.0 / 20.7, clustered 84 /
+// 77 / 79, 256 scenes 299 / 279 / 272).  Loading a pair's next tile ahead costs
+// the registers of a CTA; an L2 prefetch of it 77 -> 80.
+constexpr uint32_t kPairTiles = 16u;  // per SM
+template <uint32_t kBodies>
+constexpr uint32_t kIntegrateCtas = kBodies == 1u ? 5u : 6u;
+template <bool kP2P, uint32_t kBodies>
+__global__ void __launch_bounds__(kTile / kBodies, kIntegrateCtas<kBodies>) k_integrate(const SceneDesc *__restrict__ scenes,
                                                    const uint32_t *__restrict__ tile_scene,
                                                    float4 *__restrict__ part,
                                                    const uint4 *__restrict__ mom,
@@ -504,7 +636,7 @@ __global__ void __launch_bounds__(256, 5) k_integrate(const SceneDesc *__restric
                                                    uint4 *__restrict__ mom_next, uint32_t tiles,
                                                    const uint32_t *__restrict__ tile_list,
                                                    Counters *__restrict__ ctr, int dynamic,
-                                                   const float4 *__restrict__ near4,
+                                                   const float4 *__restrict__ near4, float minus_zero,
                                                    unsigned long long *__restrict__ stamp) {
   __shared__ DepositTable T;
   __shared__ SceneDesc S;
@@ -546,43 +678,69 @@ __global__ void __launch_bounds__(256, 5) k_integrate(const SceneDesc *__restric
   if (dynamic) grid_dependency_wait();  // its counter belongs to the tree passes
   uint32_t i = dynamic ? grab() : static_tile(k);
   uint32_t cur = 0xFFFFFFFFu;
-  // The next tile's bodies are loaded one iteration ahead.
-  float4 n0 = make_float4(0.f, 0.f, 0.f, 0.f), n1 = n0;
+  using V = std::conditional_t<kBodies == 1u, float, f32x2>;
+  V mz;
+  splat(mz, minus_zero);
+  float4 next_lo[kBodies], next_hi[kBodies];
+  auto load = [&](uint32_t tile) {
+#pragma unroll
+    for (uint32_t h = 0; h < kBodies; h++)
+      load_body(part, tile * kTile + kBodies * threadIdx.x + h, next_lo[h], next_hi[h]);
+  };
   uint32_t next_tile = i < end ? (tile_list != nullptr ? tile_list[i] : i) : 0u;
   if (i < end) {
-    load_body(part, next_tile * kTile + threadIdx.x, n0, n1);
+    load(next_tile);
     cur = tile_scene[next_tile];
     enter_scene(cur);
   }
   grid_dependency_wait();  // fields of this step are complete
   stamp_begin(stamp);
   while (i < end) {
-    const uint32_t tile = next_tile;
-    const uint32_t slot = tile * kTile + threadIdx.x;
-    float4 p0 = n0, p1 = n1;
-    const uint32_t ni = dynamic ? grab() : static_tile(++k);
-    if (ni < end) {
-      next_tile = tile_list != nullptr ? tile_list[ni] : ni;
-      load_body(part, next_tile * kTile + threadIdx.x, n0, n1);
+    const uint32_t tile = next_tile, slot = tile * kTile + kBodies * threadIdx.x;
+    float4 lo[kBodies], hi[kBodies];
+#pragma unroll
+    for (uint32_t h = 0; h < kBodies; h++) {
+      lo[h] = next_lo[h];
+      hi[h] = next_hi[h];
     }
-    i = ni;
+    i = dynamic ? grab() : static_tile(++k);
+    // One body per lane: the next tile's are loaded meanwhile; two leave no
+    // registers for that.
+    if (i < end) next_tile = tile_list != nullptr ? tile_list[i] : i;
+    if (kBodies == 1u && i < end) load(next_tile);
     // The CTA's last tile: the next step's upward pass may launch now (it
     // waits for this whole grid before reading anything); its CTAs take SM
     // slots as this grid's CTAs leave.
-    if (ni >= end) grid_dependents_may_launch();
+    if (i >= end) grid_dependents_may_launch();
     const uint32_t sc = tile_scene[tile];
     if (sc != cur) {
       enter_scene(sc);
       cur = sc;
     }
-    const bool active = slot - C.body_off < C.n;
-    uint32_t key = DepositTable::kEmpty;
-    uint32_t qx = kBiasBits, qy = kBiasBits, qz = kBiasBits;
-    if (active) {
-      integrate_body<kP2P>(S, C, p0, p1, mom, src, aux, choice, fields, kP2P ? near4 + slot : nullptr, key, qx, qy, qz);
-      store_body(part, slot, p0, p1);
+    const uint32_t body = slot - C.body_off;
+    uint32_t key[kBodies], q[kBodies][3];
+#pragma unroll
+    for (uint32_t h = 0; h < kBodies; h++) {
+      key[h] = DepositTable::kEmpty;
+      q[h][0] = q[h][1] = q[h][2] = kBiasBits;
     }
-    if (!kP2P) deposit_body<kBiasBits>(T, key, active, qx, qy, qz, mom_next);
+    if (body < C.n) {
+      integrate_bodies<kP2P>(S, C, mz, lo, hi, mom, src, aux, choice, fields, kP2P ? near4 + slot : nullptr, key, q);
+#pragma unroll
+      for (uint32_t h = 0; h < kBodies; h++) {
+        if (h == 0u || body + h < C.n)
+          store_body(part, slot + h, lo[h], hi[h]);
+        else
+          key[h] = DepositTable::kEmpty;
+      }
+    }
+    if (kBodies > 1u && i < end) load(next_tile);
+    if (!kP2P) {
+      if constexpr (kBodies == 1u)
+        deposit_body<kBiasBits>(T, key[0], key[0] != DepositTable::kEmpty, q[0][0], q[0][1], q[0][2], mom_next);
+      else
+        deposit_two<kBiasBits>(T, key[0], key[1], q[0], q[1], mom_next);
+    }
   }
   if (!kP2P) {
     __syncthreads();
@@ -1119,7 +1277,7 @@ __global__ void __launch_bounds__(256) k_deposit(const SceneDesc *__restrict__ s
       qy = (uint32_t)f2i_rn_sat(p.y * S.scale);
       qz = (uint32_t)f2i_rn_sat(p.z * S.scale);
     }
-    deposit_body<0u>(T, key, active, qx, qy, qz, moments);
+    deposit_body(T, key, active, qx, qy, qz, moments);
   }
   __syncthreads();
   T.flush(moments);
@@ -1321,7 +1479,7 @@ __global__ void __launch_bounds__(256) k_gather(const SceneDesc *__restrict__ sc
       qy = (uint32_t)f2i_rn_sat(p0.y * S.scale);
       qz = (uint32_t)f2i_rn_sat(p0.z * S.scale);
     }
-    deposit_body<0u>(T, key, active, qx, qy, qz, deposit_into);
+    deposit_body(T, key, active, qx, qy, qz, deposit_into);
   }
   __syncthreads();
   T.flush(deposit_into);
@@ -1483,11 +1641,21 @@ __global__ void __launch_bounds__(256) k_initialize(const SceneDesc *__restrict_
 
 // --------------------------------------------------------------- launches
 
-uint32_t body_ctas_per_sm() {
+template <uint32_t kBodies>
+static uint32_t integrate_ctas_per_sm() {
   int n = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_integrate<false>, kTile, 0) != cudaSuccess || n < 1)
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_integrate<false, kBodies>, kTile / kBodies, 0) !=
+          cudaSuccess ||
+      n < 1)
     n = 1;
   return (uint32_t)n;
+}
+uint32_t body_ctas_per_sm() {
+#ifdef RFMM_FAST_FLOAT
+  return integrate_ctas_per_sm<1u>();
+#else
+  return integrate_ctas_per_sm<2u>();
+#endif
 }
 
 // Persistent body-pass grid: whole waves of resident CTAs, at most one per tile.
@@ -1495,14 +1663,25 @@ static uint32_t body_grid(const LaunchCtx &L, uint32_t tiles) {
   return tiles < L.body_ctas ? tiles : L.body_ctas;
 }
 
-void launch_integrate(const LaunchCtx &L, uint32_t tiles) {
-  static const uint32_t per_sm = body_ctas_per_sm();
+template <uint32_t kBodies>
+static void launch_integrate_bodies(const LaunchCtx &L, uint32_t tiles) {
+  static const uint32_t per_sm = integrate_ctas_per_sm<kBodies>();
   const uint32_t grid = body_grid(L, tiles), wave = L.sms * per_sm;
-  launch_step_kernel(L, L.p2p ? k_integrate<true> : k_integrate<false>, dim3(grid < wave ? grid : wave),
-                     dim3(kTile), 0, L.scenes, L.tile_scene, L.part, (const uint4 *)L.mom,
-                     (const float4 *)L.src, (const float4 *)L.aux, (const uint32_t *)L.choice,
-                     (const float *)L.fields, L.mom_next, tiles, L.tile_list, L.ctr,
-                     L.integrate_dynamic ? 1 : 0, (const float4 *)L.near4, stamp_rec(L, 3u));
+  launch_step_kernel(L, L.p2p ? k_integrate<true, kBodies> : k_integrate<false, kBodies>,
+                     dim3(grid < wave ? grid : wave), dim3(kTile / kBodies), 0, L.scenes, L.tile_scene, L.part,
+                     (const uint4 *)L.mom, (const float4 *)L.src, (const float4 *)L.aux, (const uint32_t *)L.choice,
+                     (const float *)L.fields, L.mom_next, tiles, L.tile_list, L.ctr, L.integrate_dynamic ? 1 : 0,
+                     (const float4 *)L.near4, -0.0f, stamp_rec(L, 3u));
+}
+
+void launch_integrate(const LaunchCtx &L, uint32_t tiles) {
+#ifndef RFMM_FAST_FLOAT
+  if (tiles > kPairTiles * L.sms) {
+    launch_integrate_bodies<2u>(L, tiles);
+    return;
+  }
+#endif
+  launch_integrate_bodies<1u>(L, tiles);
 }
 
 // One wave of the pair-sum kernel's resident CTAs, at most one warp per unit.

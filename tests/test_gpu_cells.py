@@ -68,3 +68,24 @@ def test_steps_at_cell_and_wall_boundaries_bit_exact(rfmm_mod, oracle_mod, depth
         s.step(2)
         assert np.array_equal(s.particles().view(np.uint32), st.particles.view(np.uint32))
         assert np.array_equal(s.moments().view(np.uint32), np.asarray(st.moments).view(np.uint32))
+
+
+@pytest.mark.parametrize("n", [33, 255, 257, 4099])
+@pytest.mark.parametrize("spread", [0.01, 0.2, 1.3])
+def test_deposit_runs_bit_exact(rfmm_mod, oracle_mod, n, spread):
+    """Steps without a re-sort between them, so that leaves hold one run, many
+    short ones and single bodies, at odd counts that end inside a lane's pair:
+    states and moments equal the oracle's."""
+    O, R = oracle_mod, rfmm_mod
+    rng = np.random.default_rng(n)
+    p = np.zeros(n, R.PARTICLE_DTYPE)
+    p["pos"] = rng.normal(0.0, spread, (n, 3))
+    p["vel"] = rng.normal(0.0, 40.0 * spread, (n, 3))
+    kw = dict(gravity=1.0, softening=1e-3, dt=5e-4, depth=4)
+    st = O.OracleState(p, O.make_params(n, **kw))
+    st.step(5)
+    with R.Solver(n, R.default_params(**kw)) as s:
+        s.upload(p)
+        s.step(5)
+        assert np.array_equal(s.particles().view(np.uint32), st.particles.view(np.uint32))
+        assert np.array_equal(s.moments().view(np.uint32), np.asarray(st.moments).view(np.uint32))
