@@ -725,6 +725,8 @@ __device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, i
 // 189 contributing cells of that child, but each load touches up to 32 lines
 // and L1 bounds the pass: 112 us, 110 with packed terms, at 256 scenes of 4k
 // to 262k bodies against 100 us here; the fast variant 101 against 79.)
+// Neighbouring groups go to one CTA, whose warps then share lines: 89 us, fast
+// 71 (with six CTAs per SM launched 97 and 76).
 __device__ __forceinline__ void m2l_lanes_pass(const SceneDesc *__restrict__ scenes,
                                                const WorkItem *__restrict__ plist, uint32_t count,
                                                const uint4 *__restrict__ mom,
@@ -735,7 +737,7 @@ __device__ __forceinline__ void m2l_lanes_pass(const SceneDesc *__restrict__ sce
   // Bit u of near[axis]: tile coordinate u (0..5) lies within one cell of the
   // target's, 2 + its child bit.
   const uint32_t near_x = 7u << (1u + (c & 1u)), near_y = 7u << (1u + ((c >> 1) & 1u)), near_z = 7u << (1u + (c >> 2));
-  for (uint32_t g = blockIdx.x + gridDim.x * (threadIdx.x >> 5); g < groups; g += gridDim.x * wpb) {
+  for (uint32_t g = blockIdx.x * wpb + (threadIdx.x >> 5); g < groups; g += gridDim.x * wpb) {
     const uint32_t item = 4u * g + (lane >> 3);
     const bool valid = item < count;
     const WorkItem w = valid ? plist[item] : WorkItem{0u, 0u};
@@ -1293,7 +1295,10 @@ void launch_m2l(const LaunchCtx &L, uint32_t list_par) {
   const bool w = wide(L.m2l_lanes, L);
   auto kernel = L.m2l_compact ? (w ? k_m2l<true, true> : k_m2l<true, false>)
                               : (w ? k_m2l<false, true> : k_m2l<false, false>);
-  launch_step_kernel(L, kernel, dim3(L.m2l_ctas), dim3(256),
+  // The lane path's four CTAs per SM stay resident: more leave the last ones a
+  // wave of their own.
+  const uint32_t grid = w && L.m2l_ctas > 4u * L.sms ? 4u * L.sms : L.m2l_ctas;
+  launch_step_kernel(L, kernel, dim3(grid), dim3(256),
                      m2l_smem_bytes(L.m2l_compact), L.scenes,
                      (const WorkItem *)L.plist, L.plist_cap, L.ctr, list_par, (const uint4 *)L.mom,
                      (const float4 *)L.src, L.lfield, L.tmaps, lane_min(L.m2l_lanes, kM2LLaneAuto), -0.0f,
@@ -1308,8 +1313,6 @@ void launch_l2l_near(const LaunchCtx &L, uint32_t list_par) {
                      lane_min(L.l2l_lanes, kL2LLaneAuto), stamp_rec(L, 2u));
 }
 
-constexpr int kUpwardCarveout = 58;  // percent of the SM's shared memory: 132 KB
-
 cudaError_t configure_tree_kernels() {
   cudaError_t e = cudaSuccess;
   const std::pair<void (*)(const SceneDesc *, const WorkItem *, uint32_t, Counters *, uint32_t,
@@ -1322,15 +1325,6 @@ cudaError_t configure_tree_kernels() {
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(k.first, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)m2l_smem_bytes(k.second));
-  // The upward pass starts on SMs that integrate is leaving.  With the
-  // driver's choice (hardly any shared memory) between the many-scene launches'
-  // larger ones, every such SM has to empty before its memory is divided
-  // anew, around each early launch: 256 scenes, 20 steps, 14.9 ms with 132 KB,
-  // 15.0 with 164 KB, 16.3 to 17.2 with the driver's choice.  (One scene: no
-  // difference.  The same setting for integrate costs the 5,242,880-body
-  // step 1 % of L1.)
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_upward<true>, cudaFuncAttributePreferredSharedMemoryCarveout, kUpwardCarveout);
   return e;
 }
 
