@@ -1263,7 +1263,9 @@ void launch_wait_check(cudaStream_t stream, uint32_t polls, uint32_t *status) {
 // L2L + near).
 constexpr uint32_t kNever = 0xFFFFFFFFu;
 constexpr uint32_t kUpwardWarpAuto = 4096u;
-constexpr uint32_t kM2LLaneAuto = 16384u;
+// us, per-item / lane path: 3,086 parents 24.6 / 37.2, 5,436 37.8 / 43.5, 9,264
+// 69.0 / 57.9 (fast 22.3 / 32.0, 34.9 / 35.5, 63.3 / 46.0).
+constexpr uint32_t kM2LLaneAuto = 8192u;
 constexpr uint32_t kL2LLaneAuto = 2048u;
 static uint32_t lane_min(uint32_t mode, uint32_t automatic) {
   return mode == 0u ? kNever : (mode == 1u ? 0u : automatic);
