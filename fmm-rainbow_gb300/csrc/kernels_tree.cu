@@ -1262,11 +1262,16 @@ void launch_wait_check(cudaStream_t stream, uint32_t polls, uint32_t *status) {
 // crossovers: subtree tasks for the upward pass, listed parents for M2L and
 // L2L + near).
 constexpr uint32_t kNever = 0xFFFFFFFFu;
-constexpr uint32_t kUpwardWarpAuto = 4096u;
-// us, per-item / lane path: 3,086 parents 24.6 / 37.2, 5,436 37.8 / 43.5, 9,264
-// 69.0 / 57.9 (fast 22.3 / 32.0, 34.9 / 35.5, 63.3 / 46.0).
+// us per launch, per-item / second path.  Upward: 4,096 subtrees 25.2 to 25.8 /
+// 35.4, 6,144 35.1 / 40.0 (but the step of 12 scenes of 1,048,576 bodies 326 /
+// 323), 8,192 47.4 to 52.8 / 45.9 to 55.6, 12,288 71 to 74 / 57 to 64.  M2L: 3,086
+// parents 24.6 / 37.2, 5,436 37.8 / 43.5, 9,264 69.0 / 57.9 (fast 22.3 / 32.0, 34.9
+// / 35.5, 63.3 / 46.0).  L2L + near: 2,152 parents 9.9 / 13.5, 3,086 13.8 / 14.6,
+// 4,304 17.7 / 15.5, 5,944 23.1 / 15.8 (the step of 28 scenes of 65,536 bodies with
+// 3,766 parents 96.9 / 93.4).
+constexpr uint32_t kUpwardWarpAuto = 6144u;
 constexpr uint32_t kM2LLaneAuto = 8192u;
-constexpr uint32_t kL2LLaneAuto = 2048u;
+constexpr uint32_t kL2LLaneAuto = 3072u;
 static uint32_t lane_min(uint32_t mode, uint32_t automatic) {
   return mode == 0u ? kNever : (mode == 1u ? 0u : automatic);
 }
