@@ -302,6 +302,14 @@ __device__ __forceinline__ void biased_cells(const StepScene &C, const V (&p)[3]
 #pragma unroll
   for (int h = 0; h < kN; h++) ok[h] = max_abs3(d[0][h], d[1][h], d[2][h]) <= C.cell_margin;
 }
+// RN(RN(p scale) + kBias): the fixed-point coordinate in the sum's low bits.
+// Two roundings in every variant, as the deposit of an upload makes them.
+__device__ __forceinline__ float biased_fixed(float p, float scale, float) {
+  return __fadd_rn(__fmul_rn(p, scale), kBias);
+}
+__device__ __forceinline__ f32x2 biased_fixed(f32x2 p, float scale, f32x2 mz) {
+  return add2(mul2(p, pack2(scale, scale), mz), pack2(kBias, kBias));
+}
 __device__ __forceinline__ float biased_cell_slow(const StepScene &C, float p) {
   return (float)cell_of_unit(unit_coord(p), C.dim) + kBias;
 }
@@ -584,7 +592,7 @@ __device__ __forceinline__ void integrate_bodies(const SceneDesc &S, const StepS
 #pragma unroll
   for (int c = 0; c < 3; c++) {
     halves(t[c], u[c]);
-    halves(add2(mul(p[c], all(C.scale)), all(kBias)), b[c]);
+    halves(biased_fixed(p[c], C.scale, mz), b[c]);
   }
 #pragma unroll
   for (int h = 0; h < kN; h++) {
