@@ -1039,10 +1039,15 @@ int Engine::solve_fields() {
 }
 
 int Engine::launch_chunk(uint32_t len, bool sort_at_end) {
-  if (len == 1u && near_mode_ == kNearReference && !timeline_ && !use_lists_) {
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (len == 1u && near_mode_ == kNearReference && !timeline_ && !use_lists_ &&
+      cudaStreamIsCapturing(stream_, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone) {
     // A lone step of four launches: launched directly they chain to the work
     // before them like the steps inside a graph do, and nothing is captured
-    // for a first step (4,096 bodies, one frame: 48 us as a graph).
+    // for a first step (4,096 bodies, one frame: 48 us as a graph).  On a
+    // stream the caller is capturing it takes the graph's way, which is
+    // refused: captured launches would replay on this step's buffers, and the
+    // buffers alternate.
     enqueue_step(mcur_, lpar_, pcur_);
     if (sort_at_end) enqueue_resort(pcur_, mcur_ ^ 1u);
     RF_CK(cudaGetLastError());
@@ -1090,7 +1095,11 @@ int Engine::capture_chunk(uint32_t len, uint32_t mcur, uint32_t lpar, uint32_t p
       rec = d_stamps_ + (size_t)region * kStampSteps * kStampWordsPerStep;
     }
     cudaGraph_t g = nullptr;
-    RF_CK(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
+    const cudaError_t begun = cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal);
+    if (begun != cudaSuccess) {
+      (void)cudaGetLastError();  // reported here, not by the next call
+      return cuda_status(begun);
+    }
     if (rec != nullptr)
       cudaMemsetAsync(rec, 0, 8ull * kStampSteps * kStampWordsPerStep, stream_);
     for (uint32_t j = 0; j < len; j++)
