@@ -42,6 +42,24 @@ EncodeTiledFn get_encode_tiled() {
   return fn;
 }
 
+// Whether one device allocation holds all of [p, p + bytes).
+bool one_allocation(const void *p, size_t bytes) {
+  using AddressRangeFn = CUresult (*)(CUdeviceptr *, size_t *, CUdeviceptr);
+  static const AddressRangeFn fn = [] {
+    void *f = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPointByVersion("cuMemGetAddressRange", &f, 12000, cudaEnableDefault, &q) != cudaSuccess ||
+        q != cudaDriverEntryPointSuccess)
+      f = nullptr;
+    return reinterpret_cast<AddressRangeFn>(f);
+  }();
+  CUdeviceptr base = 0;
+  size_t size = 0;
+  const CUdeviceptr at = reinterpret_cast<CUdeviceptr>(p);
+  return fn != nullptr && fn(&base, &size, at) == CUDA_SUCCESS && at >= base && at - base <= size &&
+         bytes <= size - (at - base);
+}
+
 const StepLaunchers kExactLaunchers = {launch_upward,    launch_m2l,      launch_l2l_near,
                                        launch_integrate, launch_near_p2p, launch_accel,
                                        launch_accel_targets};
@@ -72,10 +90,14 @@ int cuda_status(cudaError_t e) {
   return RFMM_ERR_CUDA;
 }
 
-#define RF_CK(call)                                 \
-  do {                                              \
-    cudaError_t e_ = (call);                        \
-    if (e_ != cudaSuccess) return cuda_status(e_);  \
+// A failed call's error is returned, and not left for the next call to find.
+#define RF_CK(call)            \
+  do {                         \
+    cudaError_t e_ = (call);   \
+    if (e_ != cudaSuccess) {   \
+      (void)cudaGetLastError();\
+      return cuda_status(e_);  \
+    }                          \
   } while (0)
 
 const char *status_string(int status) {
@@ -915,19 +937,22 @@ int Engine::refresh_lists() {
 }
 
 // A device buffer the kernels can read or write in place: device or managed
-// memory of this device, 32-byte aligned.
-bool Engine::usable_in_place(const void *p) const {
+// memory of this device, 32-byte aligned, one allocation holding all of it.
+// Anything else goes through a copy, with the checks of the runtime: a buffer
+// that is too short is refused there.
+bool Engine::usable_in_place(const void *p, size_t bytes) const {
   cudaPointerAttributes a{};
   if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
     (void)cudaGetLastError();  // a failed attribute query leaves no error behind
     return false;
   }
   return ((a.type == cudaMemoryTypeDevice && a.device == device_) || a.type == cudaMemoryTypeManaged) &&
-         (reinterpret_cast<uintptr_t>(p) & 31u) == 0u;
+         (reinterpret_cast<uintptr_t>(p) & 31u) == 0u && one_allocation(p, bytes);
 }
 
 int Engine::upload_commit_device(const void *src, size_t bytes) {
-  if (scenes_.size() != 1u || use_lists_ || src == nullptr || bytes != 32ull * scenes_[0].n || !usable_in_place(src)) {
+  if (scenes_.size() != 1u || use_lists_ || src == nullptr || bytes != 32ull * scenes_[0].n ||
+      !usable_in_place(src, bytes)) {
     const int st = upload(0, src, bytes, cudaMemcpyDeviceToDevice);
     return st == RFMM_OK ? commit() : st;
   }
@@ -1095,11 +1120,7 @@ int Engine::capture_chunk(uint32_t len, uint32_t mcur, uint32_t lpar, uint32_t p
       rec = d_stamps_ + (size_t)region * kStampSteps * kStampWordsPerStep;
     }
     cudaGraph_t g = nullptr;
-    const cudaError_t begun = cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal);
-    if (begun != cudaSuccess) {
-      (void)cudaGetLastError();  // reported here, not by the next call
-      return cuda_status(begun);
-    }
+    RF_CK(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
     if (rec != nullptr)
       cudaMemsetAsync(rec, 0, 8ull * kStampSteps * kStampWordsPerStep, stream_);
     for (uint32_t j = 0; j < len; j++)
@@ -1218,7 +1239,7 @@ int Engine::download(uint32_t scene, int which, void *dst, size_t bytes, cudaMem
   if (which == RFMM_BUF_PARTICLES) {
     if (!committed_) return RFMM_ERR_STATE;
     LaunchCtx L = ctx(mcur_, lpar_, pcur_);
-    if (kind == cudaMemcpyDeviceToDevice && usable_in_place(dst)) {
+    if (kind == cudaMemcpyDeviceToDevice && usable_in_place(dst, bytes)) {
       // Straight into the caller's buffer; the launch also reports the error
       // word, so no copy follows.
       launch_unpermute(L, d_ids_[pcur_], static_cast<float4 *>(dst), d.tile_off, pad_tiles(d.n), nullptr, nullptr,
@@ -1237,7 +1258,7 @@ int Engine::download(uint32_t scene, int which, void *dst, size_t bytes, cudaMem
     if (!solved_) return RFMM_ERR_STATE;
     from = d_fields_ + 12ull * d.cell_off;
   }
-  if (kind == cudaMemcpyDeviceToDevice && usable_in_place(dst)) {
+  if (kind == cudaMemcpyDeviceToDevice && usable_in_place(dst, bytes)) {
     launch_copy_out(ctx(mcur_, lpar_, pcur_), from, dst, bytes, &h_ctr_->error);
     RF_CK(cudaGetLastError());
     RF_CK(cudaStreamSynchronize(stream_));

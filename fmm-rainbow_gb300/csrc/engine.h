@@ -214,7 +214,7 @@ class Engine {
   int rebuild_lists();
   int check_device_error();
   int reported_error() const;
-  bool usable_in_place(const void *p) const;
+  bool usable_in_place(const void *p, size_t bytes) const;
 
   int device_ = 0;
   int sms_ = 0;
