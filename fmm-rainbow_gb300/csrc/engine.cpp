@@ -957,6 +957,7 @@ int Engine::upload_commit_device(const void *src, size_t bytes) {
     return st == RFMM_OK ? commit() : st;
   }
   uploaded_[0] = true;
+  committed_ = false;  // until the commit is through, as after upload()
   return commit(static_cast<const float4 *>(src));
 }
 
