@@ -42,22 +42,18 @@ EncodeTiledFn get_encode_tiled() {
   return fn;
 }
 
-// Whether one device allocation holds all of [p, p + bytes).
-bool one_allocation(const void *p, size_t bytes) {
-  using AddressRangeFn = CUresult (*)(CUdeviceptr *, size_t *, CUdeviceptr);
-  static const AddressRangeFn fn = [] {
-    void *f = nullptr;
+using PointerAttributesFn = CUresult (*)(unsigned int, CUpointer_attribute *, void **, CUdeviceptr);
+
+PointerAttributesFn get_pointer_attributes() {
+  static const PointerAttributesFn fn = [] {
+    void *p = nullptr;
     cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPointByVersion("cuMemGetAddressRange", &f, 12000, cudaEnableDefault, &q) != cudaSuccess ||
+    if (cudaGetDriverEntryPointByVersion("cuPointerGetAttributes", &p, 12000, cudaEnableDefault, &q) != cudaSuccess ||
         q != cudaDriverEntryPointSuccess)
-      f = nullptr;
-    return reinterpret_cast<AddressRangeFn>(f);
+      p = nullptr;
+    return reinterpret_cast<PointerAttributesFn>(p);
   }();
-  CUdeviceptr base = 0;
-  size_t size = 0;
-  const CUdeviceptr at = reinterpret_cast<CUdeviceptr>(p);
-  return fn != nullptr && fn(&base, &size, at) == CUDA_SUCCESS && at >= base && at - base <= size &&
-         bytes <= size - (at - base);
+  return fn;
 }
 
 const StepLaunchers kExactLaunchers = {launch_upward,    launch_m2l,      launch_l2l_near,
@@ -941,13 +937,20 @@ int Engine::refresh_lists() {
 // Anything else goes through a copy, with the checks of the runtime: a buffer
 // that is too short is refused there.
 bool Engine::usable_in_place(const void *p, size_t bytes) const {
-  cudaPointerAttributes a{};
-  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
-    (void)cudaGetLastError();  // a failed attribute query leaves no error behind
-    return false;
-  }
-  return ((a.type == cudaMemoryTypeDevice && a.device == device_) || a.type == cudaMemoryTypeManaged) &&
-         (reinterpret_cast<uintptr_t>(p) & 31u) == 0u && one_allocation(p, bytes);
+  const PointerAttributesFn query = get_pointer_attributes();
+  if (query == nullptr || (reinterpret_cast<uintptr_t>(p) & 31u) != 0u) return false;
+  CUmemorytype type = static_cast<CUmemorytype>(0);
+  int managed = 0, ordinal = -1;
+  CUdeviceptr start = 0;
+  size_t size = 0;
+  CUpointer_attribute what[] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_IS_MANAGED,
+                                CU_POINTER_ATTRIBUTE_DEVICE_ORDINAL, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR,
+                                CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+  void *into[] = {&type, &managed, &ordinal, &start, &size};
+  const CUdeviceptr at = reinterpret_cast<CUdeviceptr>(p);
+  if (query(5, what, into, at) != CUDA_SUCCESS) return false;
+  if (managed == 0 && (type != CU_MEMORYTYPE_DEVICE || ordinal != device_)) return false;
+  return at >= start && at - start <= size && bytes <= size - (at - start);
 }
 
 int Engine::upload_commit_device(const void *src, size_t bytes) {
