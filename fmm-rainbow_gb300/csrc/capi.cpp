@@ -189,6 +189,11 @@ int rfmm_check_wait_timeout(rfmm_handle *h, uint32_t polls) {
   return h->engine->check_wait_timeout(polls);
 }
 
+int rfmm_check_sort_timeout(rfmm_handle *h, uint32_t polls) {
+  if (guard(h)) return RFMM_ERR_INVALID;
+  return h->engine->check_sort_timeout(polls);
+}
+
 int rfmm_device_error(rfmm_handle *h, uint32_t *code, uint32_t *info) {
   if (guard(h)) return RFMM_ERR_INVALID;
   return h->engine->device_error(code, info);

@@ -6,6 +6,8 @@
 #include <chrono>
 #include <cmath>
 #include <cstring>
+#include <memory>
+#include <new>
 #include <vector>
 
 #include "rfmm_internal.h"
@@ -1213,6 +1215,43 @@ int Engine::check_wait_timeout(uint32_t polls) {
   RF_CK(cudaStreamSynchronize(stream_));
   if (got == (uint32_t)kDevErrTmaTimeout) return RFMM_ERR_TIMEOUT;
   return got == (uint32_t)kDevErrNone ? RFMM_OK : RFMM_ERR_CUDA;
+}
+
+int Engine::check_sort_timeout(uint32_t polls) {
+  if (polls == 0u || polls > (1u << 22)) return RFMM_ERR_INVALID;
+  constexpr uint32_t kPoison = 0xA5A5A5A5u;
+  std::unique_ptr<SortWaitCheck> h(new (std::nothrow) SortWaitCheck());
+  if (h == nullptr) return RFMM_ERR_OOM;
+  void *scratch = nullptr;
+  RF_CK(cudaMalloc(&scratch, sizeof(SortWaitCheck)));
+  SortWaitCheck *d = static_cast<SortWaitCheck *>(scratch);
+  for (uint32_t i = 0; i < 3u * SortWaitCheck::kTileKeys; i++) {
+    h->keys[i] = i & 255u;
+    h->out_keys[i] = h->out_vals[i] = kPoison;
+  }
+  uint32_t error[2] = {kDevErrNone, kDevErrNone};
+  cudaError_t e = cudaSuccess;
+  // Tile 1 waits for tile 0, which never runs; then tile 2 finds tile 1 failed.
+  for (uint32_t tile = 1; tile <= 2u && e == cudaSuccess; tile++) {
+    for (uint32_t &t : h->totals) t = 3u * SortWaitCheck::kTileKeys / 256u;
+    h->state = SortState{tile, 0u, SortWaitCheck::kEpoch};
+    h->ctr = Counters{};
+    e = cudaMemcpyAsync(d, h.get(), sizeof(SortWaitCheck), cudaMemcpyHostToDevice, stream_);
+    if (e == cudaSuccess) {
+      launch_sort_wait_check(stream_, polls, d);
+      e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpyAsync(h.get(), d, sizeof(SortWaitCheck), cudaMemcpyDeviceToHost, stream_);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(stream_);
+    error[tile - 1u] = h->ctr.error;
+    launches_ += 1;
+  }
+  cudaFree(scratch);
+  RF_CK(e);
+  if (error[0] == kDevErrNone) return RFMM_OK;
+  const bool closed = error[0] == kDevErrSortTimeout && error[1] == kDevErrNone &&
+                      sort_wait_check_failed_closed(*h, kPoison);
+  return closed ? RFMM_ERR_TIMEOUT : RFMM_ERR_DEVICE;
 }
 
 int Engine::device_error(uint32_t *code, uint32_t *info) {

@@ -64,6 +64,9 @@ class Engine {
   int upload(uint32_t scene, const void *src, size_t bytes, cudaMemcpyKind kind);
   // Runs a bounded wait that cannot complete; RFMM_ERR_TIMEOUT when it gave up.
   int check_wait_timeout(uint32_t polls);
+  // The same for the sort's wait between tiles, with what a tile that gave up
+  // must leave behind.
+  int check_sort_timeout(uint32_t polls);
   // Every scene's bodies from one device buffer per scene (caller order).
   int upload_all_device(const void *const *src);
   // Every scene's buffer `which` to dst[scene]: one reorder launch, one copy

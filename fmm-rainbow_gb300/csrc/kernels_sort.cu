@@ -70,6 +70,8 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t *w
 // passes read as absent).
 constexpr uint32_t kSortOwn = 1u;   // the tile's own count
 constexpr uint32_t kSortUpTo = 2u;  // the count of every tile up to this one
+constexpr uint32_t kSortFailed = 3u;  // none: this tile, or one before it, gave up waiting
+constexpr uint32_t kSortPolls = 1u << 22;  // polls of a tile's wait for its predecessors, a few seconds
 __device__ __forceinline__ unsigned long long sort_word(uint32_t epoch, uint32_t kind, uint32_t count) {
   return ((unsigned long long)((epoch << 2) | kind) << 32) | count;
 }
@@ -79,7 +81,7 @@ __global__ void __launch_bounds__(kSortThreads) k_sort_pass(
     const uint32_t *__restrict__ keys_in, const uint32_t *__restrict__ vals_in,
     const uint32_t *__restrict__ tile_map, uint32_t *__restrict__ keys_out, uint32_t *__restrict__ vals_out,
     uint32_t n, uint32_t shift, uint32_t *__restrict__ totals, unsigned long long *__restrict__ status,
-    SortState *__restrict__ state, Counters *__restrict__ ctr) {
+    SortState *__restrict__ state, Counters *__restrict__ ctr, uint32_t max_polls) {
   constexpr uint32_t kTileKeys = kSortThreads * kItems, kAll = 0xFFFFFFFFu;
   __shared__ uint32_t s_key[kTileKeys], s_val[kTileKeys];
   __shared__ uint32_t s_cnt[kSortWarps][256];  // per warp: digit counts, then first rank in the tile
@@ -163,15 +165,16 @@ __global__ void __launch_bounds__(kSortThreads) k_sort_pass(
     const uint32_t digit0 = block_exclusive_scan(total, s_sums);
     // Look back until a tile that knows its whole prefix.  Tickets number
     // tiles in the order their CTAs began, so every predecessor is running;
-    // the wait is bounded all the same.
+    // the wait is bounded all the same, and a tile that gives up, or finds that
+    // one before it did, publishes that instead of a count and writes nothing.
     uint32_t before = 0u;
     if (tile != 0u) {
       // Four predecessors per round trip, nearest first (1 / 4 / 8 / 16 at
       // 1,048,576 bodies: 109 / 104 / 105 / 116 us per upload).
       constexpr uint32_t kBack = 4u;
       uint32_t back = tile;  // tiles [back, tile) are counted in `before`
-      bool open = true;
-      for (uint32_t polls = 0u; open;) {
+      uint32_t kind = kSortOwn;  // of the last word taken
+      for (uint32_t polls = 0u; kind == kSortOwn;) {
         unsigned long long w[kBack];
 #pragma unroll
         for (uint32_t j = 0; j < kBack; j++)
@@ -181,20 +184,20 @@ __global__ void __launch_bounds__(kSortThreads) k_sort_pass(
 #pragma unroll
         for (uint32_t j = 0; j < kBack; j++) {
           const uint32_t tag = (uint32_t)(w[j] >> 32);
-          if (open && used == j && (tag >> 2) == (epoch & 0x3FFFFFFFu) && (tag & 3u) != 0u) {
+          if (kind == kSortOwn && used == j && (tag >> 2) == (epoch & 0x3FFFFFFFu) && (tag & 3u) != 0u) {
             before += (uint32_t)w[j];
             used = j + 1u;
-            open = (tag & 3u) != kSortUpTo;
+            kind = tag & 3u;
           }
         }
         back -= used;
-        if (open && used == 0u && ++polls == 1u << 22) {
+        if (used == 0u && ++polls == max_polls) {
           if (atomicCAS(&ctr->error, 0u, (uint32_t)kDevErrSortTimeout) == 0u) ctr->error_info = tile;
-          s_stop = 1u;
-          break;
+          kind = kSortFailed;
         }
       }
-      *mine = sort_word(epoch, kSortUpTo, before + count);
+      if (kind == kSortFailed) s_stop = 1u;
+      *mine = sort_word(epoch, kind, before + count);
     }
     s_out[tid] = digit0 + before - first;
   }
@@ -249,10 +252,27 @@ int radix_sort(const LaunchCtx &L, SortScratch &s, uint32_t n, uint32_t bits, co
   for (uint32_t shift = 0; shift < bits; shift += 8u) {
     launch_step_kernel(L, pass, dim3(ntiles), dim3(kSortThreads), 0, (const uint32_t *)s.keys[cur],
                        (const uint32_t *)(shift == 0u ? nullptr : s.vals[cur]), tile_map, s.keys[cur ^ 1],
-                       s.vals[cur ^ 1], n, shift, s.totals + 256u * (shift / 8u), s.status, s.state, L.ctr);
+                       s.vals[cur ^ 1], n, shift, s.totals + 256u * (shift / 8u), s.status, s.state, L.ctr, kSortPolls);
     cur ^= 1;
   }
   return cur;
+}
+
+void launch_sort_wait_check(cudaStream_t stream, uint32_t polls, SortWaitCheck *check) {
+  static_assert(SortWaitCheck::kTileKeys == kSortThreads * kSortItemsSmall, "small tiles");
+  k_sort_pass<kSortItemsSmall><<<1, kSortThreads, 0, stream>>>(
+      check->keys, nullptr, nullptr, check->out_keys, check->out_vals, 3u * SortWaitCheck::kTileKeys, 0u,
+      check->totals, check->status, &check->state, &check->ctr, polls);
+}
+
+// What the two launches of the check must leave: tiles 1 and 2 marked failed
+// for every digit, the output as it was, and the state ready for a next pass.
+bool sort_wait_check_failed_closed(const SortWaitCheck &h, uint32_t poison) {
+  for (uint32_t i = 0; i < 3u * SortWaitCheck::kTileKeys; i++)
+    if (h.out_keys[i] != poison || h.out_vals[i] != poison) return false;
+  for (uint32_t i = 256u; i < 3u * 256u; i++)
+    if ((uint32_t)(h.status[i] >> 32) != ((SortWaitCheck::kEpoch << 2) | kSortFailed)) return false;
+  return h.state.ticket == 0u && h.state.done == 0u && h.state.epoch == SortWaitCheck::kEpoch + 1u;
 }
 
 // ------------------------------------------------ leaf counting-sort resort

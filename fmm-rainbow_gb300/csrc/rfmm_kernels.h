@@ -234,6 +234,18 @@ size_t sort_status_words(uint32_t capacity);
 // Sorts keys[0] (written by launch_keys with the same digits and tile map) over
 // `bits` low bits; returns which buffer holds the result.  Values are slots.
 int radix_sort(const LaunchCtx &L, SortScratch &s, uint32_t n, uint32_t bits, const uint32_t *tile_map = nullptr);
+// Self-check of the bounded wait inside a sort pass, on scratch of its own: a
+// launch runs the one tile that `state.ticket` numbers, of three tiles of
+// which nothing publishes tile 0's counts.
+struct SortWaitCheck {
+  static constexpr uint32_t kTileKeys = 1024u, kEpoch = 1u;
+  uint32_t keys[3u * kTileKeys], out_keys[3u * kTileKeys], out_vals[3u * kTileKeys], totals[256];
+  unsigned long long status[3u * 256u];
+  SortState state;
+  Counters ctr;
+};
+void launch_sort_wait_check(cudaStream_t stream, uint32_t polls, SortWaitCheck *check);
+bool sort_wait_check_failed_closed(const SortWaitCheck &host, uint32_t poison);
 // Leaf counting sort of every scene's bodies (part_in/ids_in -> part_out/
 // ids_out) from the leaf counts in `counts` (moments of the current
 // positions).  block_scratch: leaf_sort_blocks(max_depth) words per scene;

@@ -178,6 +178,7 @@ SIGNATURES = {
     "rfmm_batch_upload_device_all": (_i, [_vp, _vp]),
     "rfmm_batch_download_all": (_i, [_vp, _i, _vp]),
     "rfmm_check_wait_timeout": (_i, [_vp, _u32]),
+    "rfmm_check_sort_timeout": (_i, [_vp, _u32]),
     "rfmm_batch_seed_galaxy": (_i, [_vp, _u32]),
     "rfmm_batch_commit": (_i, [_vp]),
     "rfmm_batch_solve_fields": (_i, [_vp]),
@@ -388,6 +389,10 @@ class Solver:
     def check_wait_timeout(self, polls: int = 1024) -> int:
         """Run the bounded-wait self-check; returns the status code (ERR_TIMEOUT expected)."""
         return lib().rfmm_check_wait_timeout(self._h, polls)
+
+    def check_sort_timeout(self, polls: int = 1024) -> int:
+        """The same for the sort's wait between tiles."""
+        return lib().rfmm_check_sort_timeout(self._h, polls)
 
     def download_host_ptr(self, which: int, ptr: int, nbytes: int):
         _check(lib().rfmm_download(self._h, which, ptr, nbytes), "rfmm_download")

@@ -191,6 +191,11 @@ int rfmm_device_error(rfmm_handle *h, uint32_t *code, uint32_t *info);
  * Returns RFMM_ERR_TIMEOUT when the wait gave up as it must (the handle stays
  * usable and its error word is untouched), RFMM_OK never in practice. */
 int rfmm_check_wait_timeout(rfmm_handle *h, uint32_t polls);
+/* The same for the wait between the tiles of an upload's sort, on scratch of
+ * its own: a tile whose predecessor never publishes gives up, the tile after
+ * it stops as well, and neither writes.  RFMM_ERR_TIMEOUT when all that holds,
+ * RFMM_ERR_DEVICE when the wait gave up otherwise. */
+int rfmm_check_sort_timeout(rfmm_handle *h, uint32_t polls);
 
 /* Kernel kinds of rfmm_profile_steps. */
 enum rfmm_kernel_kind {
