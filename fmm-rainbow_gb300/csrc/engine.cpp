@@ -59,11 +59,11 @@ PointerAttributesFn get_pointer_attributes() {
 }
 
 const StepLaunchers kExactLaunchers = {launch_upward,    launch_m2l,      launch_l2l_near,
-                                       launch_integrate, launch_near_p2p, launch_accel,
+                                       launch_integrate, integrate_pairs, launch_near_p2p, launch_accel,
                                        launch_accel_targets};
 const StepLaunchers kFastLaunchers = {fast::launch_upward,   fast::launch_m2l,
                                       fast::launch_l2l_near, fast::launch_integrate,
-                                      fast::launch_near_p2p, fast::launch_accel,
+                                      fast::integrate_pairs, fast::launch_near_p2p, fast::launch_accel,
                                       fast::launch_accel_targets};
 
 }  // namespace
@@ -192,6 +192,7 @@ int Engine::create(const std::vector<SceneSpec> &specs, Engine **out) {
   }
   E->slots_ = body_off;
   E->tiles_ = body_off / kTile;
+  E->active_tiles_ = E->tiles_;
   E->cells_ = cell_off;
   E->tasks_ = task_off;
   // Sort key = scene rank above a Morton code of fine cells (level F >= the
@@ -599,6 +600,7 @@ LaunchCtx Engine::ctx(uint32_t mpar, uint32_t lpar, uint32_t ppar) const {
   L.m2l_ctas = (uint32_t)sms_ * tuning_.m2l_ctas_per_sm;
   L.l2l_ctas = (uint32_t)sms_ * tuning_.l2l_ctas_per_sm;
   L.integrate_dynamic = tuning_.integrate_dynamic != 0u;
+  L.integrate_pairs = pairs();
   L.m2l_compact = tuning_.m2l_compact != 0u;
   L.m2l_lanes = tuning_.m2l_lanes;
   L.l2l_lanes = tuning_.l2l_lanes;
@@ -730,6 +732,7 @@ int Engine::rebuild_lists() {
       for (uint32_t t = 0; t < (1u << (3u * d.sub_level)); t++) tasks[nk++] = d.task_off + t;
       sl[ns++] = i;
     }
+    active_tiles_ = nt;
     blk[0] = nt;
     blk[1] = nk;
     blk[2] = ns;
@@ -1100,21 +1103,25 @@ int Engine::launch_chunk(uint32_t len, bool sort_at_end) {
 
 int Engine::prepare_graphs(uint32_t max_len) {
   if (max_len == 0u || max_len > tuning_.graph_steps) return RFMM_ERR_INVALID;
+  const uint32_t active = active_tiles_;
+  const std::vector<uint32_t> loads = use_lists_ ? std::vector<uint32_t>{0u, tiles_} : std::vector<uint32_t>{active};
+  int st = RFMM_OK;
   for (uint32_t len = 1; len <= max_len; len++)
-    for (uint32_t m = 0; m < 2u; m++)
-      for (uint32_t l = 0; l < 2u; l++)
-        for (uint32_t p = 0; p < 2u; p++)
-          for (int sort = 0; sort < (resort_interval_ > 0 ? 2 : 1); sort++) {
+    for (uint32_t m = 0; m < 2u; m++)  // steps flip the moment and the list buffer together
+      for (uint32_t p = 0; p < 2u; p++)
+        for (int sort = 0; sort < (resort_interval_ > 0 ? 2 : 1); sort++)
+          for (uint32_t load : loads) {  // the lightest and the fullest take every form there is
             Graph *g = nullptr;
-            const int st = capture_chunk(len, m, l, p, sort != 0, &g);
-            if (st != RFMM_OK) return st;
+            active_tiles_ = load;
+            if (st == RFMM_OK) st = capture_chunk(len, m, m, p, sort != 0, &g);
           }
-  return RFMM_OK;
+  active_tiles_ = active;
+  return st;
 }
 
 int Engine::capture_chunk(uint32_t len, uint32_t mcur, uint32_t lpar, uint32_t pcur, bool sort_at_end,
                           Graph **out) {
-  const auto key = std::make_tuple(len, mcur, lpar, pcur, sort_at_end);
+  const auto key = std::make_tuple(len, mcur, lpar, pcur, sort_at_end, pairs());
   auto it = graphs_.find(key);
   if (it == graphs_.end()) {
     // Timeline: this graph's records, cleared by its first node.

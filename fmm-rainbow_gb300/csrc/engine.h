@@ -33,6 +33,7 @@ struct StepLaunchers {
   void (*m2l)(const LaunchCtx &, uint32_t);
   void (*l2l_near)(const LaunchCtx &, uint32_t);
   void (*integrate)(const LaunchCtx &, uint32_t);
+  bool (*integrate_pairs)(uint32_t, uint32_t);
   void (*near_p2p)(const LaunchCtx &, uint32_t);
   void (*accel)(const LaunchCtx &, const uint32_t *, float4 *, uint32_t, uint32_t);
   void (*accel_targets)(const LaunchCtx &, uint32_t, uint32_t, uint32_t, const uint32_t *,
@@ -103,8 +104,9 @@ class Engine {
   // which must come before the next step.
   int retire_many(const std::vector<uint32_t> &slots);
   int refresh_lists();
-  // Captures the step graphs of every chunk length up to max_len and every
-  // buffer parity ahead of time (serving: no capture while requests wait).
+  // Captures the step graphs of every chunk length up to max_len, every buffer
+  // parity that steps alone lead to and every form of integrate ahead of time
+  // (serving: no capture while requests wait).
   int prepare_graphs(uint32_t max_len);
   // Seconds refresh_lists spent waiting for a pinned list block's last copy.
   double list_wait_seconds() const { return list_wait_s_; }
@@ -227,6 +229,8 @@ class Engine {
   rfmm_tuning tuning_{};
   void clear_graphs();
   bool use_lists_ = false;  // serving: kernels walk the active tile/task lists
+  uint32_t active_tiles_ = 0;  // tiles of the scenes that have bodies, as the next step sees them
+  bool pairs() const { return K().integrate_pairs(active_tiles_, (uint32_t)sms_); }
   cudaStream_t stream_ = nullptr;
   cudaStream_t own_stream_ = nullptr;
 
@@ -309,7 +313,8 @@ class Engine {
   bool timeline_ = false;
   uint32_t stamp_regions_used_ = 0;
   unsigned long long *d_stamps_ = nullptr;
-  std::map<std::tuple<uint32_t, uint32_t, uint32_t, uint32_t, bool>, Graph> graphs_;
+  // By length, moment, list and particle buffers, re-sort at the end, form of integrate.
+  std::map<std::tuple<uint32_t, uint32_t, uint32_t, uint32_t, bool, bool>, Graph> graphs_;
   // The step graph of `len` steps from the given buffer parities (captured
   // and instantiated on first use).
   int capture_chunk(uint32_t len, uint32_t mcur, uint32_t lpar, uint32_t pcur, bool sort_at_end, Graph **out);

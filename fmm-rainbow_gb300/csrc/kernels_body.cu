@@ -622,8 +622,10 @@ __device__ __forceinline__ void integrate_bodies(const SceneDesc &S, const StepS
 // 63 %).  One / two, exact: 250,000 Plummer bodies 6.1 / 8.6, 524,288 11.7 /
 // 12.2 (uniform 9.45 / 9.15), 700,000 13.4 / 13.4, 1,048,576 20.4 / 18.9
 // (uniform 16.2 / 15.4), 5,242,880 clustered 83.3 / 76.6, 256 scenes 295 /
-// 279: pairs pay from about 16 tiles per SM.  The fast variant's contracted
-// chains are shorter and gain nothing from packing (clustered 71 / 73).
+// 279: pairs pay from about 16 tiles per SM.  What counts is the tiles with
+// bodies in them: a server's slots are mostly empty (one request of 250,000 bodies
+// in slots of 2^20: 5.9 / 7.6 a step).  The fast variant's contracted chains are
+// shorter and gain nothing from packing (clustered 71 / 73).
 //
 // Resident CTAs per SM: five of 256 (6 / 5: clustered 84.3 / 83.5, 256 scenes
 // 300 / 295), six of 128 (5 / 6 / 7: Plummer 21.9 / 19.0 / 20.7, clustered 84 /
@@ -1682,9 +1684,17 @@ static void launch_integrate_bodies(const LaunchCtx &L, uint32_t tiles) {
                      (const float4 *)L.near4, -0.0f, stamp_rec(L, 3u));
 }
 
+bool integrate_pairs(uint32_t tiles, uint32_t sms) {
+#ifdef RFMM_FAST_FLOAT
+  return false;
+#else
+  return tiles > kPairTiles * sms;
+#endif
+}
+
 void launch_integrate(const LaunchCtx &L, uint32_t tiles) {
 #ifndef RFMM_FAST_FLOAT
-  if (tiles > kPairTiles * L.sms) {
+  if (L.integrate_pairs) {
     launch_integrate_bodies<2u>(L, tiles);
     return;
   }

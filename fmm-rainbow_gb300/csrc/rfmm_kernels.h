@@ -63,6 +63,7 @@ struct LaunchCtx {
   uint32_t m2l_ctas;           // persistent grid of the M2L pass
   uint32_t l2l_ctas;           // persistent grid of the L2L + near pass
   bool integrate_dynamic;      // integrate CTAs grab tiles from a counter
+  bool integrate_pairs;        // integrate with two bodies per lane (integrate_pairs() below)
   bool m2l_compact;            // M2L variant that lists contributing slots first
   uint32_t m2l_lanes;          // M2L with one lane per target: 0 never, 1 always, 2 long lists
   uint32_t l2l_lanes;          // L2L + near with one lane per target: the same
@@ -122,6 +123,9 @@ cudaError_t configure_tree_kernels();
 
 // Body passes (kernels_body.cu).
 void launch_integrate(const LaunchCtx &L, uint32_t tiles);
+// Whether a step of `tiles` body tiles (the active ones, where there is a list)
+// takes two bodies per lane.
+bool integrate_pairs(uint32_t tiles, uint32_t sms);
 // kNearP2P: exact near-field pair sums of every body into L.near4.
 void launch_near_p2p(const LaunchCtx &L, uint32_t tiles);
 void launch_deposit(const LaunchCtx &L, uint4 *moments, uint32_t tiles);
@@ -218,6 +222,7 @@ void launch_upward(const LaunchCtx &L, uint32_t list_par, uint32_t tasks);
 void launch_m2l(const LaunchCtx &L, uint32_t list_par);
 void launch_l2l_near(const LaunchCtx &L, uint32_t list_par);
 void launch_integrate(const LaunchCtx &L, uint32_t tiles);
+bool integrate_pairs(uint32_t tiles, uint32_t sms);
 void launch_near_p2p(const LaunchCtx &L, uint32_t tiles);
 void launch_accel(const LaunchCtx &L, const uint32_t *ids, float4 *out, uint32_t tile_base,
                   uint32_t tiles);
