@@ -1745,8 +1745,11 @@ void launch_deposit(const LaunchCtx &L, uint4 *moments, uint32_t tiles) {
 void launch_keys(const LaunchCtx &L, const SortScratch &s, uint32_t bits, uint32_t *ids, int fresh_ids,
                  uint32_t tiles, const SceneMask *fresh, const uint32_t *tile_map, const ClearTree *clear) {
   static const SceneMask kNone{};
-  const uint32_t wave = 8u * L.sms;
-  launch_step_kernel(L, k_keys, dim3(tiles < wave ? tiles : wave), dim3(kTile), 0, L.scenes, L.tile_scene,
+  // A CTA per tile, or per 256 words to clear where those are more (255 bodies
+  // in a forced depth-6 tree: 309 us per upload with one CTA per tile, 19 now).
+  const uint32_t wave = 8u * L.sms, clears = clear != nullptr ? (clear->words + kTile - 1u) / kTile : 0u;
+  const uint32_t ctas = tiles > clears ? tiles : clears;
+  launch_step_kernel(L, k_keys, dim3(ctas < wave ? ctas : wave), dim3(kTile), 0, L.scenes, L.tile_scene,
                      (const float4 *)L.part, s.keys[0], ids, fresh_ids, tiles, fresh != nullptr ? *fresh : kNone,
                      tile_map, (bits + 7u) / 8u, s.totals, clear != nullptr ? *clear : ClearTree{});
 }
