@@ -70,7 +70,10 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t *w
 // passes read as absent).
 constexpr uint32_t kSortOwn = 1u;   // the tile's own count
 constexpr uint32_t kSortUpTo = 2u;  // the count of every tile up to this one
-constexpr uint32_t kSortFailed = 3u;  // none: this tile, or one before it, gave up waiting
+// Top bit of a count up to a tile: that tile, or one before it, gave up
+// waiting.  (Counts stay below 2^31.  As a fourth kind of word, told apart in
+// the look-back's loop, it took 0.5 us a pass at 65,536 keys.)
+constexpr uint32_t kSortFailed = 0x80000000u;
 constexpr uint32_t kSortPolls = 1u << 22;  // polls of a tile's wait for its predecessors, a few seconds
 __device__ __forceinline__ unsigned long long sort_word(uint32_t epoch, uint32_t kind, uint32_t count) {
   return ((unsigned long long)((epoch << 2) | kind) << 32) | count;
@@ -166,15 +169,15 @@ __global__ void __launch_bounds__(kSortThreads) k_sort_pass(
     // Look back until a tile that knows its whole prefix.  Tickets number
     // tiles in the order their CTAs began, so every predecessor is running;
     // the wait is bounded all the same, and a tile that gives up, or finds that
-    // one before it did, publishes that instead of a count and writes nothing.
+    // one before it did, publishes that with its count and writes nothing.
     uint32_t before = 0u;
     if (tile != 0u) {
       // Four predecessors per round trip, nearest first (1 / 4 / 8 / 16 at
       // 1,048,576 bodies: 109 / 104 / 105 / 116 us per upload).
       constexpr uint32_t kBack = 4u;
       uint32_t back = tile;  // tiles [back, tile) are counted in `before`
-      uint32_t kind = kSortOwn;  // of the last word taken
-      for (uint32_t polls = 0u; kind == kSortOwn;) {
+      bool open = true;
+      for (uint32_t polls = 0u; open;) {
         unsigned long long w[kBack];
 #pragma unroll
         for (uint32_t j = 0; j < kBack; j++)
@@ -184,20 +187,21 @@ __global__ void __launch_bounds__(kSortThreads) k_sort_pass(
 #pragma unroll
         for (uint32_t j = 0; j < kBack; j++) {
           const uint32_t tag = (uint32_t)(w[j] >> 32);
-          if (kind == kSortOwn && used == j && (tag >> 2) == (epoch & 0x3FFFFFFFu) && (tag & 3u) != 0u) {
+          if (open && used == j && (tag >> 2) == (epoch & 0x3FFFFFFFu) && (tag & 3u) != 0u) {
             before += (uint32_t)w[j];
             used = j + 1u;
-            kind = tag & 3u;
+            open = (tag & 3u) != kSortUpTo;
           }
         }
         back -= used;
-        if (used == 0u && ++polls == max_polls) {
+        if (open && used == 0u && ++polls == max_polls) {
           if (atomicCAS(&ctr->error, 0u, (uint32_t)kDevErrSortTimeout) == 0u) ctr->error_info = tile;
-          kind = kSortFailed;
+          before |= kSortFailed;
+          break;
         }
       }
-      if (kind == kSortFailed) s_stop = 1u;
-      *mine = sort_word(epoch, kind, before + count);
+      if (before >= kSortFailed) s_stop = 1u;
+      *mine = sort_word(epoch, kSortUpTo, before + count);
     }
     s_out[tid] = digit0 + before - first;
   }
@@ -271,7 +275,9 @@ bool sort_wait_check_failed_closed(const SortWaitCheck &h, uint32_t poison) {
   for (uint32_t i = 0; i < 3u * SortWaitCheck::kTileKeys; i++)
     if (h.out_keys[i] != poison || h.out_vals[i] != poison) return false;
   for (uint32_t i = 256u; i < 3u * 256u; i++)
-    if ((uint32_t)(h.status[i] >> 32) != ((SortWaitCheck::kEpoch << 2) | kSortFailed)) return false;
+    if ((uint32_t)(h.status[i] >> 32) != ((SortWaitCheck::kEpoch << 2) | kSortUpTo) ||
+        (uint32_t)h.status[i] < kSortFailed)
+      return false;
   return h.state.ticket == 0u && h.state.done == 0u && h.state.epoch == SortWaitCheck::kEpoch + 1u;
 }
 
