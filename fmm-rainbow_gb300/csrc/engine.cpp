@@ -59,11 +59,12 @@ PointerAttributesFn get_pointer_attributes() {
 }
 
 const StepLaunchers kExactLaunchers = {launch_upward,    launch_m2l,      launch_l2l_near,
-                                       launch_integrate, integrate_pairs, launch_near_p2p, launch_accel,
-                                       launch_accel_targets};
+                                       launch_integrate, integrate_pairs, integrate_resident, launch_near_p2p,
+                                       launch_accel, launch_accel_targets};
 const StepLaunchers kFastLaunchers = {fast::launch_upward,   fast::launch_m2l,
                                       fast::launch_l2l_near, fast::launch_integrate,
-                                      fast::integrate_pairs, fast::launch_near_p2p, fast::launch_accel,
+                                      fast::integrate_pairs, fast::integrate_resident,
+                                      fast::launch_near_p2p, fast::launch_accel,
                                       fast::launch_accel_targets};
 
 }  // namespace
@@ -269,7 +270,7 @@ int Engine::create(const std::vector<SceneSpec> &specs, Engine **out) {
   if (e == cudaSuccess && E->use_lists_) e = cudaEventCreateWithFlags(&E->refresh_ev_, cudaEventDisableTiming);
   if (e == cudaSuccess) e = configure_tree_kernels();
   if (e == cudaSuccess) e = fast::configure_tree_kernels();
-  if (e == cudaSuccess) E->body_limit_ = body_ctas_per_sm();  // (the fast variant caps its own grid)
+  if (e == cudaSuccess) E->body_limit_ = integrate_resident(true);  // the form with the most
   {
     rfmm_tuning t{};
     // Many scenes: the warp-per-subtree upward gains from more CTAs than stay
@@ -277,13 +278,21 @@ int Engine::create(const std::vector<SceneSpec> &specs, Engine **out) {
     // against 6: -14% at 256 scenes); one scene's grid is bounded by its
     // 512 subtrees either way.
     t.upward_ctas_per_sm = specs.size() > 1 ? 16 : 6;
-    t.m2l_ctas_per_sm = 6;
+    t.m2l_ctas_per_sm = specs.size() > 1 ? 4 : 6;  // as many as stay resident (see m2l_lanes_pass)
     t.l2l_ctas_per_sm = 5;
     t.integrate_ctas_per_sm = E->body_limit_;
     t.integrate_dynamic = 0;
     t.resort_interval = 16u;
     t.graph_steps = 16;
-    t.pdl = 1;
+    // Early launches shorten a step of many small scenes (us, with / without: 8
+    // scenes of 4,096 bodies 18.8 / 20.7, 64 of 16,384 49 / 53, 32 of 65,536 103 /
+    // 106, 56 of 65,536 162 / 162).  From about 96 tiles per SM every pass fills
+    // the device for long, and a waiting launch at times takes its SMs while
+    // their shared memory is divided for its predecessor and runs at a fraction
+    // of its occupancy (64 of 65,536 221 / 195 and 202 / 176, 128 of 65,536 335 /
+    // 322 on average, 20 of 262,144 145 / 148, 20 steps of 256 of 4k to 262k
+    // 16.3 to 17.2 / 14.7 ms).
+    t.pdl = specs.size() > 1 && !E->use_lists_ && E->tiles_ > 96u * (uint32_t)E->sms_ ? 0 : 1;
     // The compacting M2L variant evaluates only the contributing stencil
     // slots; measured faster for one scene and for many.
     t.m2l_compact = 1u;
@@ -536,7 +545,13 @@ int Engine::autotune(uint32_t steps_per_trial, rfmm_tuning *best) {
         case 0: values = {2, 4, 6, 8, 16}; break;
         case 1: values = {2, 4, 6}; break;
         case 2: values = {2, 4, 5, 8}; break;
-        case 3: for (uint32_t v = 1; v <= body_limit_; v++) values.push_back(v); break;
+        case 3: {
+          // Beyond what stays resident of this engine's form a value changes nothing.
+          const uint32_t resident = std::min(body_limit_, K().integrate_resident(pairs()));
+          for (uint32_t v = 1; v <= resident; v++)
+            if (v != std::min(cur.integrate_ctas_per_sm, resident)) values.push_back(v);
+          break;
+        }
         case 4: values = {0, 1}; break;
         case 5: values = {0, 1}; break;
         case 6: values = {4, 8, 16, 32}; break;
@@ -609,15 +624,7 @@ LaunchCtx Engine::ctx(uint32_t mpar, uint32_t lpar, uint32_t ppar) const {
   L.tile_list = use_lists_ ? d_tile_list_ : nullptr;
   L.task_list = use_lists_ ? d_task_list_ : nullptr;
   L.scene_list = use_lists_ ? d_scene_list_ : nullptr;
-  // Early launches shorten a step of many small scenes (us, with / without: 8
-  // scenes of 4,096 bodies 18.8 / 20.7, 64 of 16,384 49 / 53, 32 of 65,536 103 /
-  // 106, 56 of 65,536 162 / 162).  From about 96 tiles per SM every pass fills
-  // the device for long, and a waiting launch at times takes its SMs while
-  // their shared memory is divided for its predecessor and runs at a fraction
-  // of its occupancy (64 of 65,536 221 / 195 and 202 / 176, 128 of 65,536 335 /
-  // 322 on average, 20 of 262,144 145 / 148, 20 steps of 256 of 4k to 262k
-  // 16.3 to 17.2 / 14.7 ms).
-  L.pdl = pdl_ && !(L.many_scenes && !use_lists_ && tiles_ > 96u * (uint32_t)sms_);
+  L.pdl = pdl_;
   L.p2p = near_mode_ == kNearP2P;
   L.pos4 = d_pos4_;
   L.near4 = d_near4_;

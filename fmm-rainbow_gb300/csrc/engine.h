@@ -34,6 +34,7 @@ struct StepLaunchers {
   void (*l2l_near)(const LaunchCtx &, uint32_t);
   void (*integrate)(const LaunchCtx &, uint32_t);
   bool (*integrate_pairs)(uint32_t, uint32_t);
+  uint32_t (*integrate_resident)(bool);
   void (*near_p2p)(const LaunchCtx &, uint32_t);
   void (*accel)(const LaunchCtx &, const uint32_t *, float4 *, uint32_t, uint32_t);
   void (*accel_targets)(const LaunchCtx &, uint32_t, uint32_t, uint32_t, const uint32_t *,

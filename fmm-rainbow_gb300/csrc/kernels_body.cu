@@ -1660,12 +1660,11 @@ static uint32_t integrate_ctas_per_sm() {
     n = 1;
   return (uint32_t)n;
 }
-uint32_t body_ctas_per_sm() {
-#ifdef RFMM_FAST_FLOAT
-  return integrate_ctas_per_sm<1u>();
-#else
-  return integrate_ctas_per_sm<2u>();
+uint32_t integrate_resident(bool pairs) {
+#ifndef RFMM_FAST_FLOAT
+  if (pairs) return integrate_ctas_per_sm<2u>();
 #endif
+  return integrate_ctas_per_sm<1u>();
 }
 
 // Persistent body-pass grid: whole waves of resident CTAs, at most one per tile.

@@ -726,7 +726,8 @@ __device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, i
 // and L1 bounds the pass: 112 us, 110 with packed terms, at 256 scenes of 4k
 // to 262k bodies against 100 us here; the fast variant 101 against 79.)
 // Neighbouring groups go to one CTA, whose warps then share lines: 89 us, fast
-// 71 (with six CTAs per SM launched 97 and 76).
+// 71 with the four CTAs per SM that stay resident, the default of an engine of
+// several scenes (six, of which the last ones get a wave of their own: 97 and 76).
 __device__ __forceinline__ void m2l_lanes_pass(const SceneDesc *__restrict__ scenes,
                                                const WorkItem *__restrict__ plist, uint32_t count,
                                                const uint4 *__restrict__ mom,
@@ -1302,10 +1303,7 @@ void launch_m2l(const LaunchCtx &L, uint32_t list_par) {
   const bool w = wide(L.m2l_lanes, L);
   auto kernel = L.m2l_compact ? (w ? k_m2l<true, true> : k_m2l<true, false>)
                               : (w ? k_m2l<false, true> : k_m2l<false, false>);
-  // The lane path's four CTAs per SM stay resident: more leave the last ones a
-  // wave of their own.
-  const uint32_t grid = w && L.m2l_ctas > 4u * L.sms ? 4u * L.sms : L.m2l_ctas;
-  launch_step_kernel(L, kernel, dim3(grid), dim3(256),
+  launch_step_kernel(L, kernel, dim3(L.m2l_ctas), dim3(256),
                      m2l_smem_bytes(L.m2l_compact), L.scenes,
                      (const WorkItem *)L.plist, L.plist_cap, L.ctr, list_par, (const uint4 *)L.mom,
                      (const float4 *)L.src, L.lfield, L.tmaps, lane_min(L.m2l_lanes, kM2LLaneAuto), -0.0f,

@@ -135,7 +135,7 @@ int setup_device(int dev, DeviceState &st) {
   if (e != cudaSuccess) return cuda_rc(e);
   st.scratch = S;
   st.sms = prop.multiProcessorCount;
-  st.body_ctas = (uint32_t)st.sms * body_ctas_per_sm();
+  st.body_ctas = (uint32_t)st.sms * integrate_resident(true);
   st.ready.store(true, std::memory_order_release);
   return RFMM_OK;
 }

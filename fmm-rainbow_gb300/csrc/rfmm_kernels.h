@@ -126,6 +126,7 @@ void launch_integrate(const LaunchCtx &L, uint32_t tiles);
 // Whether a step of `tiles` body tiles (the active ones, where there is a list)
 // takes two bodies per lane.
 bool integrate_pairs(uint32_t tiles, uint32_t sms);
+uint32_t integrate_resident(bool pairs);  // CTAs per SM (one 256-body tile each) of that form
 // kNearP2P: exact near-field pair sums of every body into L.near4.
 void launch_near_p2p(const LaunchCtx &L, uint32_t tiles);
 void launch_deposit(const LaunchCtx &L, uint4 *moments, uint32_t tiles);
@@ -176,7 +177,6 @@ void launch_upload_scenes(const LaunchCtx &L, float4 *part, uint32_t tile_base, 
 // Self-check of the bounded kernel wait: *status (device) receives
 // kDevErrTmaTimeout when a wait that cannot complete gives up after `polls`.
 void launch_wait_check(cudaStream_t stream, uint32_t polls, uint32_t *status);
-uint32_t body_ctas_per_sm();  // resident CTAs per SM of integrate (one 256-body tile each)
 // FMM acceleration + potential per body of tiles [tile_base, +tiles), caller order.
 void launch_accel(const LaunchCtx &L, const uint32_t *ids, float4 *out, uint32_t tile_base,
                   uint32_t tiles);
@@ -223,6 +223,7 @@ void launch_m2l(const LaunchCtx &L, uint32_t list_par);
 void launch_l2l_near(const LaunchCtx &L, uint32_t list_par);
 void launch_integrate(const LaunchCtx &L, uint32_t tiles);
 bool integrate_pairs(uint32_t tiles, uint32_t sms);
+uint32_t integrate_resident(bool pairs);
 void launch_near_p2p(const LaunchCtx &L, uint32_t tiles);
 void launch_accel(const LaunchCtx &L, const uint32_t *ids, float4 *out, uint32_t tile_base,
                   uint32_t tiles);
@@ -230,7 +231,6 @@ void launch_accel_targets(const LaunchCtx &L, uint32_t scene, uint32_t tile_base
                           const uint32_t *ids, uint32_t *slot_of, const uint32_t *targets,
                           uint32_t nt, float4 *out);
 cudaError_t configure_tree_kernels();
-uint32_t body_ctas_per_sm();
 }  // namespace fast
 
 // LSD radix sort of (key, value) pairs, 8-bit digits (kernels_sort.cu).

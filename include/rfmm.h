@@ -298,13 +298,16 @@ int rfmm_render_device(rfmm_handle *h, const rfmm_render_params *params, void *d
  * steps. */
 typedef struct rfmm_tuning {
   uint32_t upward_ctas_per_sm;    /* persistent upward grid, 1..16 */
-  uint32_t m2l_ctas_per_sm;       /* persistent M2L grid, 1..6 */
+  uint32_t m2l_ctas_per_sm;       /* persistent M2L grid, 1..6 (default 6; 4 with several scenes) */
   uint32_t l2l_ctas_per_sm;       /* persistent L2L + near grid, 1..8 */
-  uint32_t integrate_ctas_per_sm; /* persistent integrate grid, 1..resident limit */
+  uint32_t integrate_ctas_per_sm; /* persistent integrate grid, 1..resident limit (a form of the
+                                   * kernel of which fewer stay resident launches those) */
   uint32_t integrate_dynamic;     /* 0: interleaved tiles per CTA, 1: tiles from a counter */
   uint32_t resort_interval;       /* steps between resident-order refreshes, 0 = never */
   uint32_t graph_steps;           /* steps per captured CUDA graph, 1..64 */
-  uint32_t pdl;                   /* programmatic dependent launch between step kernels */
+  uint32_t pdl;                   /* programmatic dependent launch between step kernels
+                                   * (default 1; 0 for batches above 96 tiles of 256 bodies
+                                   * per SM) */
   uint32_t m2l_compact;           /* 1 (default): M2L lists each child's contributing slots
                                    * first; 0: every stencil slot, in chunks */
   uint32_t m2l_lanes;             /* M2L with one lane per target, four parents per warp:
