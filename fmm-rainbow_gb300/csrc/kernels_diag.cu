@@ -1,7 +1,9 @@
 // FP64 diagnostics: the direct-sum force reference on sampled targets and
 // compensated energy / momentum reductions.  FP64 is used only here; the
 // solver itself is binary32 throughout.  Both reductions run in a fixed order
-// (per-thread sums, then blocks in index order), so they are deterministic.
+// (the direct sum's splits in index order; the diagnostics' strided sums of a
+// warp's lanes joined pairwise, per CTA and then over the CTAs), so they are
+// deterministic.
 #include <cuda_runtime.h>
 
 #include "rfmm_kernels.h"
@@ -15,7 +17,7 @@ constexpr uint32_t kDsThreads = 256u;
 // hardware estimate y of 1/sqrt(r2) and the first terms of
 // y^3 (1 - e)^(-3/2), e = 1 - r2 y^2: six operations instead of the division,
 // square root and two products (about 19).  The first dropped term,
-// 35/16 e^3, is below 2^-56; the rounding of y^2 largely cancels between e
+// 35/16 e^3, is below 2^-55; the rounding of y^2 largely cancels between e
 // and y^3.  Error over 2^22 values of r2 in 2^-60..2^20, in units of 2^-53:
 // rms 0.6, largest 2.0 (the division form 1.9 and 6.2).  Infinite and zero r2
 // give NaN; with them every term was NaN before too (0 * inf).

@@ -20,7 +20,8 @@
 // With histogram, scan and scatter launches per pass and separate fills of the
 // tree buffers before -> now, upload with sort and deposit, us: 4,096 bodies
 // 91 -> 18, 65,536 99 -> 25, 250,000 107 -> 43, 1,048,576 147 -> 104,
-// 5,242,880 539 -> 432.
+// 5,242,880 539 -> 432; with the caller's buffer read in place and what else
+// k_gather says, 18, 22, 37, 78 and 306.
 #include <cuda_runtime.h>
 
 #include "rfmm_device.cuh"

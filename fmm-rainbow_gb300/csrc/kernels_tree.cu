@@ -1269,7 +1269,8 @@ constexpr uint32_t kNever = 0xFFFFFFFFu;
 // parents 24.6 / 37.2, 5,436 37.8 / 43.5, 9,264 69.0 / 57.9 (fast 22.3 / 32.0, 34.9
 // / 35.5, 63.3 / 46.0).  L2L + near: 2,152 parents 9.9 / 13.5, 3,086 13.8 / 14.6,
 // 4,304 17.7 / 15.5, 5,944 23.1 / 15.8 (the step of 28 scenes of 65,536 bodies with
-// 3,766 parents 96.9 / 93.4).
+// 3,766 parents 96.9 / 93.4).  What decides is the work per SM: on this GPU's 152
+// the lines lie at 40 subtrees, 54 and 20 parents for each.
 constexpr uint32_t kUpwardWarpAuto = 6144u;
 constexpr uint32_t kM2LLaneAuto = 8192u;
 constexpr uint32_t kL2LLaneAuto = 3072u;
