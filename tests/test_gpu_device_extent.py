@@ -62,3 +62,28 @@ def test_short_device_buffer_is_refused_and_handle_stays_usable(rfmm_mod):
     finally:
         for m in made:
             rt.cudaFree(C.c_void_p(m))
+
+
+@pytest.mark.parametrize("n", [257, 30001])
+def test_managed_buffers_are_taken(rfmm_mod, n):
+    """Managed memory goes the way of device memory, whatever its size."""
+    pytest.importorskip("torch")
+    R = rfmm_mod
+    from rfmm import scenes
+    p = scenes.plummer(n, seed=77)
+    with R.Solver(n) as s:
+        s.upload(p)
+        s.step(2)
+        want = s.particles()
+    rt, at = C.CDLL("libcudart.so.13"), C.c_void_p()
+    assert rt.cudaMallocManaged(C.byref(at), C.c_size_t(32 * n), C.c_uint(1)) == 0
+    try:
+        C.memmove(at.value, p.ctypes.data, 32 * n)
+        with R.Solver(n) as s:
+            s.upload_device(at.value, 32 * n)
+            s.step(2)
+            s.download_device(R.BUF_PARTICLES, at.value, 32 * n)
+        got = np.frombuffer(C.string_at(at.value, 32 * n), np.uint8)
+        assert np.array_equal(got, want.view(np.uint8))
+    finally:
+        rt.cudaFree(at)
